@@ -94,8 +94,13 @@ constexpr int kHostFirstChunkEvent = kHostFirstRangeEvent + kHostRanges;
 constexpr int kHostOrganizedEvent = kHostFirstChunkEvent + kHostPosChunks;
 constexpr int kHostEvents = kHostOrganizedEvent + 1;
 // device counters in big_count: big voxels, density tasks, tasks taken, then the
-// deferred particles of the whole force pass and of each host-entry range
-constexpr int kCounters = 4 + (kHostRanges > kPipeRanges ? kHostRanges : kPipeRanges);
+// deferred particles of the whole force pass and of each host-entry range,
+// then the tasks of the second task list and those of it taken
+constexpr int kTcCounter = 4 + (kHostRanges > kPipeRanges ? kHostRanges : kPipeRanges);
+constexpr int kCounters = kTcCounter + 2;
+// contexts of sparse and dense scenes: voxels of at most this many particles go
+// to k_density_tc, the others to k_density_wc
+constexpr int kTcVoxel = 48;
 
 struct SphgbCtx {
     int device = 0;
@@ -108,6 +113,7 @@ struct SphgbCtx {
     int v_total_ref = 0;       // reference layout
     int layout = 0;            // step layout: 0 all row-major, 1 all tiled, 2 mixed
     bool any_pipe = false;
+    bool uncapped = false;     // some scene's cap is beyond kListCap
     std::vector<SceneDev> h_scenes;
     std::vector<int32_t> h_pbegin;
     SceneDev* d_scenes = nullptr;       // step layout
@@ -202,6 +208,30 @@ struct SphgbCtx {
     cudaStream_t host_stream3 = nullptr, host_stream4 = nullptr;
     cudaEvent_t pipe_ev[3 + 2 * kPipeRanges] = {};
     std::map<int, cudaGraphExec_t> graphs;
+
+    // Which density pass takes the step's tasks: k_density_tc those of sparse
+    // scenes (the tiled ones: 1.00 ms against 1.15 with k_density_wc on the
+    // 4,194,304-particle box, 73 against 90 us at 262,144) and of scenes
+    // without a cap (27 us against 330 at 32,768, where k_density_wc walks one
+    // thread per particle); k_density_wc those of dense scenes, where its homes
+    // skip voxels one by one (203 against 256 us on the 262,144-particle pipe).
+    // Contexts of both kinds split their tasks by voxel and run both.
+    enum DensityPass { kPassTc, kPassWc, kPassBoth };
+    DensityPass density_pass() const {
+        if (layout == 1 || uncapped) return kPassTc;
+        return layout == 2 ? kPassBoth : kPassWc;
+    }
+    TaskLists task_lists() const {
+        TaskLists t;
+        t.list = tasks;
+        t.count = big_count + 1;
+        if (density_pass() == kPassBoth) {
+            t.tc_last = tasks + (n - 1);
+            t.tc_count = big_count + kTcCounter;
+            t.tc_max = kTcVoxel;
+        }
+        return t;
+    }
 
     Launch launch(cudaStream_t st, bool ref_layout = false) const {
         Launch L;
@@ -331,8 +361,12 @@ int build_scene(const SphgbSceneParams& p, int n_pipe_rows_total, SceneDev& d,
     d.h_d = hd;
     const double h2 = hd * hd;  // exact
     d.h2 = (float)h2;
+    d.inv_h2 = 1.0f / d.h2;
     d.h2_lo = round_down_f(h2 * (1.0 - std::ldexp(1.0, -18)));
     d.h2_hi = round_up_f(h2 * (1.0 + std::ldexp(1.0, -18)));
+    const double us = (double)(float)(1.0 / std::max({(double)d.vs[0], (double)d.vs[1], (double)d.vs[2]}));
+    d.u_scale = (float)us;
+    d.u_h2 = (float)(hd * us * hd * us);
     d.cull2 = round_up_f((double)d.h2_hi * (1.0 + std::ldexp(1.0, -8)));
     const double pi = 3.141592653589793;
     // normalised kernel constants (config.py:27-29 times the power of h the
@@ -679,7 +713,7 @@ cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 int enqueue_organize(SphgbCtx* c, const Launch& L, const float4* pos, const float4* vel,
                      const int32_t* pid, const double* pos64, float4* pos_o, float4* vel_o,
                      int32_t* pid_o, double* pos64_o, int32_t* vstart, int32_t* vcount,
-                     cudaEvent_t* ev = nullptr, bool with_tasks = false, bool hashed = false) {
+                     cudaEvent_t* ev = nullptr, TaskLists tasks = TaskLists{}, bool hashed = false) {
     cudaStream_t st = L.stream;
     if (!hashed) {   // else the caller cleared vcount and the counters and hashed every particle
         if (L.v_total > 0) SPHGB_CUDA(cudaMemsetAsync(vcount, 0, sizeof(int32_t) * L.v_total, st));
@@ -694,8 +728,7 @@ int enqueue_organize(SphgbCtx* c, const Launch& L, const float4* pos, const floa
     SPHGB_CUDA(launch_sort_big(L, c->big_list, c->big_count, vstart, vcount, c->tmp_pid));
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[2], st));
     SPHGB_CUDA(launch_rank_gather(L, c->cell, c->slot, pid, c->tmp_pid, vstart, vcount, pos, vel, pos64,
-                                  pos_o, vel_o, pid_o, pos64_o, with_tasks ? c->tasks : nullptr,
-                                  with_tasks ? c->big_count + 1 : nullptr));
+                                  pos_o, vel_o, pid_o, pos64_o, tasks));
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[3], st));
     return SPHGB_OK;
 }
@@ -762,14 +795,25 @@ int enqueue_step(SphgbCtx* c, cudaStream_t st, cudaEvent_t* ev = nullptr,
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[0], st));
     const float4* vel_in = vel_ready ? nullptr : c->velA;   // null: gathered after density
     const float4* vel_s = vel_ready ? nullptr : c->velB;
+    const bool warp = c->density_variant == SPHGB_DENSITY_WARP;
+    const TaskLists lists = c->task_lists();
     int rc = enqueue_organize(c, L, c->posA, vel_in, c->pidA, p64A, c->posB, c->velB, c->pidB,
-                              p64B, c->vstart, c->vcount, ev ? ev + 1 : nullptr, true, hashed);
+                              p64B, c->vstart, c->vcount, ev ? ev + 1 : nullptr, lists, hashed);
     if (rc) return rc;
     if (organized) SPHGB_CUDA(cudaEventRecord(organized, st));
-    if (c->density_variant == SPHGB_DENSITY_WARP)
-        SPHGB_CUDA(launch_density_wc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                     c->nbr, c->tasks, c->big_count + 1, c->big_count + 2));
-    else
+    if (warp) {
+        const SphgbCtx::DensityPass pass = c->density_pass();
+        if (pass == SphgbCtx::kPassTc)
+            SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
+                                         c->nbr, lists.list, 1, lists.count, c->big_count + 2));
+        else
+            SPHGB_CUDA(launch_density_wc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
+                                         c->nbr, lists.list, lists.count, c->big_count + 2));
+        if (pass == SphgbCtx::kPassBoth)
+            SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
+                                         c->nbr, lists.tc_last, -1, lists.tc_count,
+                                         lists.tc_count + 1));
+    } else
         SPHGB_CUDA(launch_density(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
                                   c->nbr));
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[5], st));
@@ -896,6 +940,8 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
     c->n_pipe_rows = n_pipe_rows_total;
     c->n_chunks = (int)chunks.size();
     c->any_pipe = any_pipe;
+    c->uncapped = false;
+    for (const SceneDev& d : c->h_scenes) c->uncapped |= d.cap > kListCap;
     // the caller binds (new) state and outputs for the new layout
     c->bound = false;
     c->nbr_valid = false;
@@ -1407,8 +1453,11 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
     // sort (the velocities follow bucket by bucket: gathered into slot order
     // by the density buckets themselves, or for the first buckets by a kernel
     // of their own on st3)
+    TaskLists whole;
+    whole.list = c->tasks;
+    whole.count = c->big_count + 1;
     int rc = enqueue_organize(c, L, c->posA, nullptr, c->pidA, p64A, c->posB, c->velB, c->pidB,
-                              p64B, c->vstart, c->vcount, nullptr, true, true);
+                              p64B, c->vstart, c->vcount, nullptr, whole, true);
     if (rc) return rc;
     SPHGB_CUDA(cudaEventRecord(e_org, st));
     // st3 after the sort and the velocity upload: the gathers and the
@@ -1449,6 +1498,8 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
     vrows.vel_out = c->velB;
     for (int b = 0; b < kPipeK; ++b) {
         if (b == kPipeGathered) SPHGB_CUDA(cudaStreamWaitEvent(st, e_vel, 0));
+        // k_density_wc, also for sparse scenes: in short launches beside the
+        // force buckets k_density_tc measured 3.06 ms per call against 2.98
         SPHGB_CUDA(launch_density_wc(L, c->posB, nullptr, c->vstart, c->vcount, c->rho, c->fin,
                                      c->nbr, c->tasks_b, pi + b, pi + 2 * kPipeK + b,
                                      pi + 4 * kPipeK + b,

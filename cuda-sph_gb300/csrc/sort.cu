@@ -283,7 +283,7 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
               const float4* __restrict__ vel, const double* __restrict__ pos64,
               float4* __restrict__ pos_out, float4* __restrict__ vel_out,
               int32_t* __restrict__ pid_out, double* __restrict__ pos64_out,
-              int2* __restrict__ tasks, int32_t* __restrict__ task_count, int big_voxel,
+              TaskLists tasks, int big_voxel,
               const int32_t* __restrict__ slot, const int32_t* __restrict__ pbegin, int n_scenes,
               const int32_t* __restrict__ step_limit, const int32_t* __restrict__ scene_step) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -327,7 +327,12 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
         r = lo;
     }
     const int d = st + r;
-    if (tasks && (r % kTaskRun) == 0) tasks[atomicAdd(task_count, 1)] = make_int2(vid, d);
+    if (tasks.list && (r % kTaskRun) == 0) {
+        if (c <= tasks.tc_max)
+            tasks.tc_last[-atomicAdd(tasks.tc_count, 1)] = make_int2(vid, d);
+        else
+            tasks.list[atomicAdd(tasks.count, 1)] = make_int2(vid, d);
+    }
     pid_out[d] = p;
     pos_out[d] = __ldg(pos + s);
     if (vel) vel_out[d] = __ldg(vel + s);   // null: velocities gathered later
@@ -391,13 +396,12 @@ cudaError_t launch_rank_gather(const Launch& L, const int32_t* cell, const int32
                                const int32_t* pid, const int32_t* tmp_pid, const int32_t* vstart,
                                const int32_t* vcount, const float4* pos, const float4* vel,
                                const double* pos64, float4* pos_out, float4* vel_out,
-                               int32_t* pid_out, double* pos64_out, int2* tasks,
-                               int32_t* task_count) {
+                               int32_t* pid_out, double* pos64_out, TaskLists tasks) {
     if (L.n == 0) return cudaSuccess;
     const int b = L.sort_block;
     k_rank_gather<<<(L.n + b - 1) / b, b, 0, L.stream>>>(L.n, cell, pid, tmp_pid, vstart, vcount,
                                                          pos, vel, pos64, pos_out, vel_out,
-                                                         pid_out, pos64_out, tasks, task_count,
+                                                         pid_out, pos64_out, tasks,
                                                          L.big_voxel, slot, L.pbegin, L.n_scenes,
                                                          L.step_limit, L.scene_step);
     return cudaGetLastError();

@@ -55,6 +55,8 @@ struct SceneDev {
     // tiled, else dims[0], dims[1]) as multiply-shift reciprocals (see Udiv)
     uint32_t div_m[2];
     int32_t div_s[2];
+    // k_density_tc: 1 / h2, 1 / largest voxel side, and (h * u_scale)^2
+    float inv_h2, u_scale, u_h2;
 };
 
 // floor(n / d) for 0 <= n < 2^31 and a divisor 1 <= d < 2^31 given as
@@ -99,6 +101,23 @@ __device__ __forceinline__ int scene_of(int s, const int32_t* __restrict__ pbegi
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
         if (__ldg(pbegin + mid) <= s) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// the same by a whole warp, s the same in every lane: a 32-way search, one round
+// of loads per factor of 32 scenes instead of one per factor of two
+__device__ __forceinline__ int scene_of_warp(int s, const int32_t* __restrict__ pbegin,
+                                             int n_scenes) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = n_scenes;
+    while (len > 1) {
+        const int step = (len + 31) >> 5, at = lane * step;
+        const unsigned m =
+            __ballot_sync(0xffffffffu, at < len && __ldg(pbegin + lo + at) <= s);
+        const int k = __popc(m) - 1;     // pbegin[lo] <= s: lane 0 is always in
+        lo += k * step;
+        len = min(step, len - k * step);
     }
     return lo;
 }
@@ -444,6 +463,64 @@ __device__ __forceinline__ void stg256(float4* p, const float4& a, const float4&
                  : "memory");
 }
 
+// ---- force inputs ----------------------------------------------------------
+// Force inputs of particle s: fin[2s] = (x, y, z, p/rho^2), fin[2s + 1] =
+// (vx, vy, vz, 1/rho), one 32-byte record that the force pass reads per
+// neighbour instead of three separate arrays.  With vel null only the first
+// half is written; k_gather_vel writes the second once the velocities are in.
+// first half of a force record: position and p / rho^2
+__device__ __forceinline__ float4 force_record_a(const float4& pi, const SceneDev& sc, float r) {
+    const float p = sc.k * (r - sc.rho0);
+    return make_float4(pi.x, pi.y, pi.z, p / (r * r));
+}
+
+__device__ __forceinline__ void write_force_inputs(int s, const float4& pi, const SceneDev& sc,
+                                                   const float4* __restrict__ vel, float r,
+                                                   float4* __restrict__ fin) {
+    const float4 a = force_record_a(pi, sc, r);
+    if (vel) {
+        const float4 v = __ldg(vel + s);
+        stg256(fin + 2 * s, a, make_float4(v.x, v.y, v.z, 1.0f / r));
+    } else {
+        fin[2 * s] = a;
+    }
+}
+
+// squared distance with the walk's arithmetic (within())
+__device__ __forceinline__ float dist2(const float4& a, const float4& b) {
+    const float dx = __fsub_rn(a.x, b.x);
+    const float dy = __fsub_rn(a.y, b.y);
+    const float dz = __fsub_rn(a.z, b.z);
+    float d2 = __fmul_rn(dx, dx);
+    d2 = __fmaf_rn(dy, dy, d2);
+    return __fmaf_rn(dz, dz, d2);
+}
+
+// Bit k (k = 9 (dx + 1) + 3 (dy + 1) + dz + 1, the walk order) is set when walk
+// voxel k of voxel (vx, vy, vz) may hold a particle within h of p: the same
+// box-distance test as walk(), against the widened
+// bound cull2.
+__device__ __forceinline__ unsigned reach_mask(const float4& p, int vx, int vy, int vz,
+                                               const SceneDev& sc) {
+    const float fx = p.x - (float)vx * sc.vs[0];
+    const float fy = p.y - (float)vy * sc.vs[1];
+    const float fz = p.z - (float)vz * sc.vs[2];
+    const float gx[3] = {fx * fx, 0.0f, (sc.vs[0] - fx) * (sc.vs[0] - fx)};
+    const float gy[3] = {fy * fy, 0.0f, (sc.vs[1] - fy) * (sc.vs[1] - fy)};
+    const float gz[3] = {fz * fz, 0.0f, (sc.vs[2] - fz) * (sc.vs[2] - fz)};
+    unsigned m = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const float gxy = gx[a] + gy[b];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if (!(gxy + gz[c] > sc.cull2)) m |= 1u << (9 * a + 3 * b + c);
+        }
+    return m;
+}
+
 // ---- neighbour list --------------------------------------------------------
 // Neighbours (other than self) of every particle in walk order, recorded by
 // the density pass and read by the force pass.  One row per particle:
@@ -538,15 +615,25 @@ cudaError_t launch_sort_big(const Launch& L, const int32_t* big_list, const int3
 // Density tasks: one (voxel, first slot) entry per run of up to kTaskRun
 // sorted slots of a voxel; a warp of the density pass takes one task at a time.
 constexpr int kTaskRun = 16;
-// tasks (optional): one (voxel, first slot) entry per run of up to kTaskRun
-// sorted slots of a voxel, appended at task_count.  tmp_pid must be 16-byte aligned
-// with 4 entries of room past n (the rank count reads it in aligned quads).
+// A task in a voxel of at most tc_max particles goes to the list that ends at
+// tc_last (entry t at tc_last[-t]); the others to the list from `list` on.
+// Both share one array: there are no more tasks than particles.  list null:
+// no tasks.
+struct TaskLists {
+    int2* list = nullptr;
+    int32_t* count = nullptr;
+    int2* tc_last = nullptr;
+    int32_t* tc_count = nullptr;
+    int tc_max = 0;      // one list
+};
+// tmp_pid must be 16-byte aligned with 4 entries of room past n (the rank
+// count reads it in aligned quads).
 cudaError_t launch_rank_gather(const Launch& L, const int32_t* cell, const int32_t* slot,
                                const int32_t* pid, const int32_t* tmp_pid, const int32_t* vstart,
                                const int32_t* vcount, const float4* pos, const float4* vel,
                                const double* pos64, float4* pos_out, float4* vel_out,
-                               int32_t* pid_out, double* pos64_out, int2* tasks = nullptr,
-                               int32_t* task_count = nullptr);
+                               int32_t* pid_out, double* pos64_out,
+                               TaskLists tasks = TaskLists{});
 // fin (optional, with vel): the force inputs of each particle, two float4
 // per particle: (x, y, z, p/rho^2) and (vx, vy, vz, 1/rho)
 cudaError_t launch_density(const Launch& L, const float4* pos, const float4* vel,
@@ -561,6 +648,11 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
                               float4* fin, NbrList nbr, const int2* tasks,
                               const int32_t* task_count, int32_t* task_next,
                               const int32_t* task_offset = nullptr, VelRows vrows = VelRows{});
+// the same on the tensor cores; task t is at tasks[t * dir]
+cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
+                              const int32_t* vstart, const int32_t* vcount, float* rho,
+                              float4* fin, NbrList nbr, const int2* tasks, int dir,
+                              const int32_t* task_count, int32_t* task_next);
 // k_gather_vel over the slots of a bucket of density tasks
 cudaError_t launch_gather_vel_tasks(const Launch& L, const int32_t* pid, const int2* tasks,
                                     const int32_t* task_count, const int32_t* task_offset,

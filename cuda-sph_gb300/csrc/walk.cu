@@ -25,27 +25,6 @@ inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
 // order (the set every later kernel of the step uses), one row per particle,
 // nbr.idx[s * kListCap + k]; nbr.count[s] = their number, or -1 when more
 // than kListCap (the force pass then walks again).
-// Force inputs of particle s: fin[2s] = (x, y, z, p/rho^2), fin[2s + 1] =
-// (vx, vy, vz, 1/rho), one 32-byte record that the force pass reads per
-// neighbour instead of three separate arrays.  With vel null only the first
-// half is written; k_gather_vel writes the second once the velocities are in.
-// first half of a force record: position and p / rho^2
-__device__ __forceinline__ float4 force_record_a(const float4& pi, const SceneDev& sc, float r) {
-    const float p = sc.k * (r - sc.rho0);
-    return make_float4(pi.x, pi.y, pi.z, p / (r * r));
-}
-
-__device__ __forceinline__ void write_force_inputs(int s, const float4& pi, const SceneDev& sc,
-                                                   const float4* __restrict__ vel, float r,
-                                                   float4* __restrict__ fin) {
-    const float4 a = force_record_a(pi, sc, r);
-    if (vel) {
-        const float4 v = __ldg(vel + s);
-        stg256(fin + 2 * s, a, make_float4(v.x, v.y, v.z, 1.0f / r));
-    } else {
-        fin[2 * s] = a;
-    }
-}
 
 // One particle's density by a thread-private walk: the walk records neighbour
 // slots in row[k * stride] (k < kListCap), the sum runs afterwards in walk
@@ -126,17 +105,8 @@ k_density(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegi
                          &s_list[0][threadIdx.x], kBlock);
 }
 
-// squared distance with the walk's arithmetic (within() in sphgb_internal.cuh)
-__device__ __forceinline__ float dist2(const float4& a, const float4& b) {
-    const float dx = __fsub_rn(a.x, b.x);
-    const float dy = __fsub_rn(a.y, b.y);
-    const float dz = __fsub_rn(a.z, b.z);
-    float d2 = __fmul_rn(dx, dx);
-    d2 = __fmaf_rn(dy, dy, d2);
-    return __fmaf_rn(dz, dz, d2);
-}
-
-// Warp-cooperative density pass of the step.  One warp per task: up to
+// Warp-cooperative density pass of the step of dense scenes, and of the
+// pipelined host order (sparse scenes: density_tc.cu).  One warp per task: up to
 // kTaskRun particles of one voxel (tasks listed by the rank-gather).  The 27
 // walk voxels of that voxel are laid end to end in walk order; each batch of
 // 96 candidates is loaded coalesced, three per lane (a candidate's slot found
@@ -158,31 +128,6 @@ constexpr int kWcList = kListCap;       // accepted neighbours per particle, sel
 constexpr int kWcPerLane = 3;           // candidates per lane in one batch
 constexpr int kWcBatch = 32 * kWcPerLane;
 constexpr int kWcCullMin = 4 * kWcBatch;  // walks longer than this skip unreachable batches
-
-// Bit k (k = 9 (dx + 1) + 3 (dy + 1) + dz + 1, the walk order) is set when walk
-// voxel k of voxel (vx, vy, vz) may hold a particle within h of p: the same
-// box-distance test as walk() in sphgb_internal.cuh, against the widened
-// bound cull2.
-__device__ __forceinline__ unsigned reach_mask(const float4& p, int vx, int vy, int vz,
-                                               const SceneDev& sc) {
-    const float fx = p.x - (float)vx * sc.vs[0];
-    const float fy = p.y - (float)vy * sc.vs[1];
-    const float fz = p.z - (float)vz * sc.vs[2];
-    const float gx[3] = {fx * fx, 0.0f, (sc.vs[0] - fx) * (sc.vs[0] - fx)};
-    const float gy[3] = {fy * fy, 0.0f, (sc.vs[1] - fy) * (sc.vs[1] - fy)};
-    const float gz[3] = {fz * fz, 0.0f, (sc.vs[2] - fz) * (sc.vs[2] - fz)};
-    unsigned m = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const float gxy = gx[a] + gy[b];
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                if (!(gxy + gz[c] > sc.cull2)) m |= 1u << (9 * a + 3 * b + c);
-        }
-    return m;
-}
 
 // Per warp.  An accepted entry is its slot and its squared distance (int
 // bits), the distance the candidate loop decided on, so the density term
@@ -320,19 +265,18 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const unsigned lt = (1u << lane) - 1u;
     const int n_tasks = *task_count;
     if (task_offset) tasks += *task_offset;   // one bucket of a bucketed task list
-    // Each warp takes its next task from a counter when it is done with the
-    // last one: the cost of a task varies with its voxel's neighbourhood, and
-    // a fixed share per warp left warps idle at the end of the pass (15 % of
-    // its time on the 4M box).
-    auto next_task = [&]() {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(task_next, 1);
-        return __shfl_sync(full, t, 0);
-    };
-    for (int t = next_task(); t < n_tasks; t = next_task()) {
+    // A warp's first task is its own number; each later one comes from a
+    // counter (the cost of a task varies with its voxel's neighbourhood, and a
+    // fixed share per warp left warps idle at the end of the pass, 15 % of its
+    // time on the 4M box).
+    const int n_warps = gridDim.x * kWcWarps;
+    int next = blockIdx.x * kWcWarps + (threadIdx.x >> 5);
+    for (;;) {
+        const int t = __shfl_sync(full, next, 0);    // uniform, also to the compiler
+        if (t >= n_tasks) break;
         const int2 task = tasks[t];
         const int vid = task.x, d0 = task.y;
-        const SceneDev& sc = scenes[scene_of(d0, pbegin, n_scenes)];
+        const SceneDev& sc = scenes[scene_of_warp(d0, pbegin, n_scenes)];
         const int vst = __ldg(vstart + vid), vc = __ldg(vcount + vid);
         const int c_t = min(kTaskRun, vst + vc - d0);
         const int s = d0 + lane;
@@ -352,6 +296,7 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
                     fin[2 * s + 1] = make_float4(v.x, v.y, v.z, 1.0f / rho[s]);
                 }
             }
+            if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
             __syncwarp();
             continue;
         }
@@ -485,6 +430,7 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             }
         }
         __syncwarp();
+        if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
     }
 }
 
@@ -953,8 +899,11 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
                               const int32_t* task_count, int32_t* task_next,
                               const int32_t* task_offset, VelRows vrows) {
     if (L.n == 0) return cudaSuccess;
-    // persistent grid: up to 4 blocks of 8 warps per SM, warps take tasks in turn
-    int blocks = (L.n + 32 * kWcWarps - 1) / (32 * kWcWarps);
+    // persistent grid: up to 4 blocks of 8 warps per SM, warps take tasks in
+    // turn; small scenes get about a warp per task, so that the tasks spread
+    // over the SMs (a task's latency is most of their pass: 8,192 particles
+    // 33 -> 17 us against one warp per 32 particles)
+    int blocks = (L.n + 8 * kWcWarps - 1) / (8 * kWcWarps);
     const int top = device_sm_count() * 4;
     if (blocks > top) blocks = top;
     // the velocity gather is its own instantiation: the step's kernel stays as it is
