@@ -363,17 +363,20 @@ __device__ inline bool pipe_is_out(const double* p, const PipeView& P, int seg, 
     return hh > r;
 }
 
-// solve_collision, util_kernels.py:182-204 with the helpers of :80-179
+// solve_collision, util_kernels.py:182-204 with the helpers of :80-179.
+// FP64 arithmetic is what bounds the wall response, so the lengths and the
+// angle that several of the helpers compute from the same values are computed
+// once (equal operands, equal bits).
 __device__ inline void pipe_solve_collision(double* p, double* v, const PipeView& P, int seg) {
     const double r0 = P.at(seg, 3), r1 = P.at(seg + 1, 3);
     // calc_edge_vector :152-171
-    double yn = __dsub_rn(p[1], P.at(seg, 1)), zn = __dsub_rn(p[2], P.at(seg, 2));
-    double hh = __dsqrt_rn(__dadd_rn(__dmul_rn(yn, yn), __dmul_rn(zn, zn)));
+    const double yn = __dsub_rn(p[1], P.at(seg, 1)), zn = __dsub_rn(p[2], P.at(seg, 2));
+    const double hh = __dsqrt_rn(__dadd_rn(__dmul_rn(yn, yn), __dmul_rn(zn, zn)));
     double first[3], second[3], edge[3];
     first[0] = P.at(seg, 0);
     second[0] = P.at(seg + 1, 0);
     for (int a = 1; a < 3; ++a) {
-        double q = __ddiv_rn(__dsub_rn(p[a], P.at(seg, a)), hh);
+        const double q = __ddiv_rn(a == 1 ? yn : zn, hh);
         first[a] = __dmul_rn(q, r0);
         second[a] = __dmul_rn(q, r1);
     }
@@ -387,33 +390,36 @@ __device__ inline void pipe_solve_collision(double* p, double* v, const PipeView
     cr[0] = __dsub_rn(__dmul_rn(edge[1], pv[2]), __dmul_rn(edge[2], pv[1]));
     cr[1] = __dsub_rn(__dmul_rn(edge[2], pv[0]), __dmul_rn(edge[0], pv[2]));
     cr[2] = __dsub_rn(__dmul_rn(edge[0], pv[1]), __dmul_rn(edge[1], pv[0]));
-    const double dd = __ddiv_rn(len3(cr), len3(edge));
+    const double dd = __ddiv_rn(len3(cr), el);
     const double sin_a = __dsqrt_rn(__dsub_rn(1.0, __dmul_rn(cos_a, cos_a)));
     const double d_to = __ddiv_rn(dd, __dadd_rn(sin_a, 0.001));
     const double dtc = __ddiv_rn(-d_to, sl);
     double cp[3];
     for (int a = 0; a < 3; ++a) cp[a] = __dadd_rn(p[a], __dmul_rn(v[a], dtc));
+    double svl = sl;        // length of the reflected velocity
     if (r0 == r1) {
         v[1] = -v[1];
         v[2] = -v[2];
-    } else {  // calc_summary_vector :88-94
-        const double ll = len3(edge), pl = len3(v);
-        const double c = __ddiv_rn(dot3(edge, v), __dmul_rn(ll, pl));
-        double sv[3];
-        for (int a = 0; a < 3; ++a)
-            sv[a] = __dmul_rn(__dmul_rn(__ddiv_rn(__dmul_rn(2.0, edge[a]), ll), c), pl);
-        for (int a = 0; a < 3; ++a) v[a] = __dsub_rn(sv[a], v[a]);
+    } else {  // calc_summary_vector :88-94, whose cosine is cos_a
+        for (int a = 0; a < 3; ++a) {
+            const double sv =
+                __dmul_rn(__dmul_rn(__ddiv_rn(__dmul_rn(2.0, edge[a]), el), cos_a), sl);
+            v[a] = __dsub_rn(sv, v[a]);
+        }
+        svl = len3(v);
     }
     double w[3];
     for (int a = 0; a < 3; ++a) w[a] = __dsub_rn(p[a], cp[a]);
     const double way = len3(w);
-    const double svl = len3(v);
     for (int a = 0; a < 3; ++a) p[a] = __dadd_rn(cp[a], __ddiv_rn(__dmul_rn(v[a], way), svl));
 }
 
 // collision_kernel (base_kernels.py:56-72) with put_particle_at_pipe_begin
 // (:101-113) and rand_position_inside_pipe (:116-127); respawn uniforms from
-// Philox keyed by (seed, particle id) with counter (draw, step).
+// Philox keyed by (seed, particle id) with counter (draw, step).  Particles
+// reflected at the inlet and particles inside a segment meet the wall in one
+// place: as two calls, the lanes of a warp that mixes them took the FP64
+// response one group after the other.
 __device__ inline void pipe_collide(double* p, double* v, const PipeView& P, uint64_t seed,
                                     uint32_t pid, uint32_t step) {
     int seg = pipe_find_segment(p, P);
@@ -421,7 +427,7 @@ __device__ inline void pipe_collide(double* p, double* v, const PipeView& P, uin
         if (p[0] < 0.0) {
             p[0] = -p[0];
             v[0] = -v[0];
-            if (pipe_is_out(p, P, 0, nullptr)) pipe_solve_collision(p, v, P, 0);
+            seg = 0;
         } else {
             p[0] = 0.0;
             int s = pipe_find_segment(p, P);
@@ -435,9 +441,8 @@ __device__ inline void pipe_collide(double* p, double* v, const PipeView& P, uin
             p[1] = __dadd_rn(P.at(0, 1), __dmul_rn(r, cs));
             p[2] = __dadd_rn(P.at(0, 2), __dmul_rn(r, sn));
         }
-    } else if (pipe_is_out(p, P, seg, nullptr)) {
-        pipe_solve_collision(p, v, P, seg);
     }
+    if (seg >= 0 && pipe_is_out(p, P, seg, nullptr)) pipe_solve_collision(p, v, P, seg);
 }
 
 // ---- 256-bit global accesses ----------------------------------------------
