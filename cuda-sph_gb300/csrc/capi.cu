@@ -98,6 +98,8 @@ constexpr int kHostEvents = kHostOrganizedEvent + 1;
 // then the tasks of the second task list and those of it taken
 constexpr int kTcCounter = 4 + (kHostRanges > kPipeRanges ? kHostRanges : kPipeRanges);
 constexpr int kCounters = kTcCounter + 2;
+constexpr size_t kCountersPad = 64;      // ints; what follows stays 128-byte aligned
+static_assert(kCounters <= (int)kCountersPad, "counters");
 // contexts of sparse and dense scenes: voxels of at most this many particles go
 // to k_density_tc, the others to k_density_wc
 constexpr int kTcVoxel = 48;
@@ -127,8 +129,11 @@ struct SphgbCtx {
     int32_t* slot = nullptr;
     int32_t* tmp_pid = nullptr;
     int32_t* vstart = nullptr;
+    // one buffer that a step clears with one memset: the counters (big_count),
+    // the scan's status words, the voxel counts
+    int32_t* counts = nullptr;
     int32_t* vcount = nullptr;
-    int32_t* tile_sums = nullptr;
+    unsigned long long* scan_status = nullptr;
     float4* posB = nullptr;
     float4* velB = nullptr;
     int32_t* pidB = nullptr;
@@ -175,8 +180,8 @@ struct SphgbCtx {
     struct {
         size_t scenes = 0, scenes_ref = 0, pbegin = 0, pipe = 0, cell = 0, slot_of = 0, slot = 0, tmp_pid = 0,
                vstart = 0,
-               vcount = 0, tile_sums = 0, posB = 0, velB = 0, pidB = 0, fin = 0, big_list = 0,
-               big_count = 0, rare = 0, tasks = 0, nbr_idx = 0, nbr_count = 0, pos64B = 0, chunks = 0,
+               counts = 0, posB = 0, velB = 0, pidB = 0, fin = 0, big_list = 0,
+               rare = 0, tasks = 0, nbr_idx = 0, nbr_count = 0, pos64B = 0, chunks = 0,
                partials = 0;
     } cap;
     // tuning (sphgb_ctx_set_tuning)
@@ -272,9 +277,9 @@ void free_ctx(SphgbCtx* c) {
     if (!c) return;
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
     void* ptrs[] = {c->d_scenes, c->d_scenes_ref, c->d_pbegin, c->d_pipe, c->cell, c->slot_of, c->slot, c->tmp_pid,
-                    c->vstart, c->vcount, c->tile_sums, c->posB, c->velB, c->pidB,
+                    c->vstart, c->counts, c->posB, c->velB, c->pidB,
                     c->pos64B, c->fin, c->owned, c->stage, c->d_chunks, c->d_partials,
-                    c->big_list, c->big_count, c->rare, c->nbr.idx, c->nbr.count, c->tasks,
+                    c->big_list, c->rare, c->nbr.idx, c->nbr.count, c->tasks,
                     c->d_check};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -708,6 +713,17 @@ inline int blocks(int n, int b = kBlock) { return (n + b - 1) / b; }
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// clears the counters, the scan's status words and the voxel counts (the
+// context's own, or a caller's table)
+int clear_counts(SphgbCtx* c, int32_t* vcount, int v_total, cudaStream_t st) {
+    const size_t head = (size_t)(c->vcount - c->counts);
+    const size_t own = vcount == c->vcount ? (size_t)v_total : 0;
+    SPHGB_CUDA(cudaMemsetAsync(c->counts, 0, sizeof(int32_t) * (head + own), st));
+    if (vcount != c->vcount && v_total > 0)
+        SPHGB_CUDA(cudaMemsetAsync(vcount, 0, sizeof(int32_t) * v_total, st));
+    return SPHGB_OK;
+}
+
 // hash + scan + scatter + big-voxel sort + rank-gather: state (any order) ->
 // voxel-sorted copy and voxel table
 int enqueue_organize(SphgbCtx* c, const Launch& L, const float4* pos, const float4* vel,
@@ -715,13 +731,13 @@ int enqueue_organize(SphgbCtx* c, const Launch& L, const float4* pos, const floa
                      int32_t* pid_o, double* pos64_o, int32_t* vstart, int32_t* vcount,
                      cudaEvent_t* ev = nullptr, TaskLists tasks = TaskLists{}, bool hashed = false) {
     cudaStream_t st = L.stream;
-    if (!hashed) {   // else the caller cleared vcount and the counters and hashed every particle
-        if (L.v_total > 0) SPHGB_CUDA(cudaMemsetAsync(vcount, 0, sizeof(int32_t) * L.v_total, st));
-        SPHGB_CUDA(cudaMemsetAsync(c->big_count, 0, kCounters * sizeof(int32_t), st));
+    if (!hashed) {   // else the caller cleared the counts and hashed every particle
+        const int rc = clear_counts(c, vcount, L.v_total, st);
+        if (rc) return rc;
         SPHGB_CUDA(launch_hash_count(L, pos, c->cell, c->slot, vcount));
     }
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[0], st));
-    SPHGB_CUDA(launch_scan(L, vcount, vstart, c->tile_sums, scan_tiles(L.v_total)));
+    SPHGB_CUDA(launch_scan(L, vcount, vstart, c->scan_status, scan_tiles(L.v_total)));
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[1], st));
     SPHGB_CUDA(launch_scatter(L, c->cell, c->slot, pid, vstart, vcount, c->tmp_pid, c->big_list,
                               c->big_count));
@@ -736,7 +752,8 @@ int enqueue_organize(SphgbCtx* c, const Launch& L, const float4* pos, const floa
 // force + integrate + wall pass of the step (after the density pass), over
 // all slots, or over a range of particles in original order when range is
 // given (see PidRange)
-int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int range_index) {
+int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int range_index,
+                   bool advance = false) {
     const bool sep = c->out_pos != nullptr;
     double* p64B = c->any_pipe ? c->pos64B : nullptr;
     float4* pos_o = sep ? c->out_pos : c->posA;
@@ -756,7 +773,7 @@ int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int rang
     else
         SPHGB_CUDA(launch_integrate(L, c->posB, c->velB, c->rho, c->fin, c->pidB, p64B, c->vstart,
                                     c->vcount, c->scene_step, c->nbr, pos_o, vel_o, pid_o, p64_o,
-                                    nullptr, rare));
+                                    nullptr, rare, advance ? c->scene_step : nullptr));
     return SPHGB_OK;
 }
 
@@ -824,8 +841,11 @@ int enqueue_step(SphgbCtx* c, cudaStream_t st, cudaEvent_t* ev = nullptr,
     }
     c->nbr_valid = true;
     if (!with_forces) return SPHGB_OK;
-    rc = enqueue_forces(c, L, nullptr, 0);
-    if (rc) return rc;
+    // the last force launch counts the step, unless something after it still
+    // reads the counters (pipe scenes have one force launch, which draws from them)
+    const bool counted = !c->any_pipe && !c->checks && !ev;
+    rc = enqueue_forces(c, L, nullptr, 0, counted);
+    if (rc || counted) return rc;
     rc = enqueue_checks(c, st);
     if (rc) return rc;
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[6], st));
@@ -900,14 +920,13 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
     rc = rc ? rc : ensure(&c->slot, k.slot, N);
     rc = rc ? rc : ensure(&c->tmp_pid, k.tmp_pid, N + 4);   // + 4: see k_rank_gather
     rc = rc ? rc : ensure(&c->vstart, k.vstart, V);
-    rc = rc ? rc : ensure(&c->vcount, k.vcount, V);
-    rc = rc ? rc : ensure(&c->tile_sums, k.tile_sums, (size_t)n_tiles);
+    const size_t head = kCountersPad + (((size_t)n_tiles * 2 + 31) & ~(size_t)31);
+    rc = rc ? rc : ensure(&c->counts, k.counts, head + V);
     rc = rc ? rc : ensure(&c->posB, k.posB, N);
     rc = rc ? rc : ensure(&c->velB, k.velB, N);
     rc = rc ? rc : ensure(&c->pidB, k.pidB, N);
     rc = rc ? rc : ensure(&c->fin, k.fin, 2 * N);
     rc = rc ? rc : ensure(&c->big_list, k.big_list, N / kMinBigVoxel + 1);
-    rc = rc ? rc : ensure(&c->big_count, k.big_count, kCounters);
     rc = rc ? rc : ensure(&c->rare, k.rare, N);
     rc = rc ? rc : ensure(&c->tasks, k.tasks, N);
     rc = rc ? rc : ensure(&c->nbr.idx, k.nbr_idx, (size_t)kListCap * N);
@@ -937,6 +956,9 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
     int n_tiled = 0;
     for (const SceneDev& d : c->h_scenes) n_tiled += d.tiled;
     c->layout = n_tiled == 0 ? 0 : (n_tiled == n_scenes ? 1 : 2);
+    c->big_count = c->counts;
+    c->scan_status = reinterpret_cast<unsigned long long*>(c->counts + kCountersPad);
+    c->vcount = c->counts + head;
     c->n_pipe_rows = n_pipe_rows_total;
     c->n_chunks = (int)chunks.size();
     c->any_pipe = any_pipe;
@@ -1446,8 +1468,10 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
     cudaEvent_t e_org = c->pipe_ev[0], e_bk = c->pipe_ev[1], e_dep = c->pipe_ev[2];
     cudaEvent_t* e_bucket = c->pipe_ev + 3;
     cudaEvent_t* e_range = c->pipe_ev + 3 + kPipeK;
-    const Launch L = c->launch(st);
-    const Launch L3 = c->launch(st3);
+    Launch L = c->launch(st), L3 = c->launch(st3);
+    // blocks that wait for the density bucket before theirs would hold the SM
+    // slots that the force buckets take meanwhile
+    L.chained = L3.chained = false;
     double* p64A = c->any_pipe ? c->pos64A : nullptr;
     double* p64B = c->any_pipe ? c->pos64B : nullptr;
     // sort (the velocities follow bucket by bucket: gathered into slot order
@@ -1665,9 +1689,10 @@ static int host_entry(SphgbCtx* ctx, const double* h_pos, const double* h_vel,
     // (particle order).  Results are the same bits as the one-stream sequence.
     SPHGB_CUDA(cudaEventRecord(e_start, st));
     SPHGB_CUDA(cudaStreamWaitEvent(st2, e_start, 0));
-    if (ctx->v_total > 0)
-        SPHGB_CUDA(cudaMemsetAsync(ctx->vcount, 0, sizeof(int32_t) * ctx->v_total, st));
-    SPHGB_CUDA(cudaMemsetAsync(ctx->big_count, 0, kCounters * sizeof(int32_t), st));
+    {
+        const int rc = clear_counts(ctx, ctx->vcount, ctx->v_total, st);
+        if (rc) return rc;
+    }
     {
         const Launch L = ctx->launch(st);
         // parts start on whole warps (the hash aggregates its atomics per warp)
@@ -2128,7 +2153,7 @@ struct NoAllocScratch {
     SceneDev scene;
     int32_t pbegin[2];
     int32_t counters[2];
-    int32_t tile_sums[kNoAllocMaxTiles];
+    unsigned long long scan_status[kNoAllocMaxTiles];
     int32_t cell[kNoAllocMaxParticles];
     int32_t slot[kNoAllocMaxParticles];
     alignas(16) int32_t tmp_pid[kNoAllocMaxParticles + 4];   // + 4: see k_rank_gather
@@ -2147,6 +2172,7 @@ NoAllocScratch* g_noalloc_addr[kNoAllocMaxDevices] = {};
 // are copied when the launch is enqueued, so no host buffer has to outlive
 // this call (a memcpy from the caller's stack would read it later).
 __global__ void k_noalloc_setup(NoAllocScratch* S, SceneDev scene, int n) {
+    for (int i = threadIdx.x; i < kNoAllocMaxTiles; i += blockDim.x) S->scan_status[i] = 0;
     if (threadIdx.x == 0) {
         S->scene = scene;
         S->pbegin[0] = 0;
@@ -2216,7 +2242,7 @@ extern "C" int sphgb_organize_voxels_noalloc(const SphgbSceneParams* scene, cons
     cudaStream_t st = as_stream(stream);
     // the scene descriptor and the counters live in the shared array too: a
     // later call overwrites them, so calls that overlap on the GPU race
-    k_noalloc_setup<<<1, 32, 0, st>>>(S, d, n);
+    k_noalloc_setup<<<1, 256, 0, st>>>(S, d, n);
     SPHGB_CUDA(cudaGetLastError());
     const int v_total = d.v_count + 1;
     SPHGB_CUDA(cudaMemsetAsync(d_voxel_count, 0, sizeof(int32_t) * v_total, st));
@@ -2235,7 +2261,7 @@ extern "C" int sphgb_organize_voxels_noalloc(const SphgbSceneParams* scene, cons
     L.stream = st;
     const float4* pos = reinterpret_cast<const float4*>(d_pos);
     SPHGB_CUDA(launch_hash_count(L, pos, S->cell, S->slot, d_voxel_count));
-    SPHGB_CUDA(launch_scan(L, d_voxel_count, d_voxel_start, S->tile_sums, scan_tiles(v_total)));
+    SPHGB_CUDA(launch_scan(L, d_voxel_count, d_voxel_start, S->scan_status, scan_tiles(v_total)));
     SPHGB_CUDA(launch_scatter(L, S->cell, S->slot, d_pid, d_voxel_start, d_voxel_count, S->tmp_pid,
                               S->big_list, &S->counters[0]));
     SPHGB_CUDA(launch_sort_big(L, S->big_list, &S->counters[0], d_voxel_start, d_voxel_count,

@@ -382,7 +382,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const int lane = threadIdx.x & 31;
     TcShared& S = sh[threadIdx.x >> 5];
     const unsigned lt = (1u << lane) - 1u;
-    const int n_tasks = *task_count;
+    const int n_tasks = *grid_wait(task_count);
     // A warp's first task is its own number; each later one comes from a
     // counter (the cost of a task varies with its voxel's neighbourhood, and a
     // fixed share per warp left warps idle at the end of the pass, 15 % of its
@@ -392,7 +392,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     for (;;) {
         const int t = __shfl_sync(full, next, 0);    // uniform, also to the compiler
         if (t >= n_tasks) break;
-        const int2 task = tasks[t * dir];
+        const int2 task = after_wait(tasks)[t * dir];
         if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
         const int vid = task.x, d0 = task.y;
         const SceneDev& sc = scenes[scene_of_warp(d0, pbegin, n_scenes)];
@@ -586,10 +586,9 @@ cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* 
     // tasks spread over the SMs (a task's latency is most of their pass)
     const int blocks = std::min((L.n + 8 * kTcWarps - 1) / (8 * kTcWarps), device_sm_count() * 6);
     auto kernel = L.layout == 1 ? k_density_tc<1> : L.layout == 2 ? k_density_tc<2> : k_density_tc<0>;
-    kernel<<<blocks, kTcWarps * 32, 0, L.stream>>>(L.scenes, L.pbegin, L.n_scenes, L.n, pos, vel,
-                                                   vstart, vcount, rho, fin, nbr, tasks, dir,
-                                                   task_count, task_next);
-    return cudaGetLastError();
+    return launch_chained(kernel, blocks, kTcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
+                          L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, dir, task_count,
+                          task_next);
 }
 
 }  // namespace sphgb

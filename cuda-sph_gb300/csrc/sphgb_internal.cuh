@@ -94,6 +94,29 @@ __host__ __device__ __forceinline__ int voxel_index(int x, int y, int z, int til
     return x + y * d0 + z * d0 * d1;
 }
 
+// ---- chained launches (launch_chained) --------------------------------------
+// Waits until the grids before this one are complete and their writes visible,
+// and lets the grid after this one be set up.  `v`, a value that the kernel's
+// addresses or loads derive from, passes through: a load of constant data
+// (ld.global.nc), which the compiler may move past a memory clobber, cannot be
+// moved ahead of the wait when its address depends on it.
+template <class T>
+__device__ __forceinline__ T grid_wait(T v) {
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "a register or a register pair");
+    if constexpr (sizeof(T) == 4)
+        asm volatile("griddepcontrol.wait;" : "+r"(v)::"memory");
+    else
+        asm volatile("griddepcontrol.wait;" : "+l"(v)::"memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return v;
+}
+// a pointer that loads after grid_wait go through
+template <class T>
+__device__ __forceinline__ T* after_wait(T* p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+
 // ---- scene lookup ---------------------------------------------------------
 // pbegin has n_scenes + 1 entries (prefix of particle counts).
 __device__ __forceinline__ int scene_of(int s, const int32_t* __restrict__ pbegin, int n_scenes) {
@@ -591,6 +614,7 @@ struct Launch {
     int big_voxel = 64;         // voxels above this many members are sorted per block
     int layout = 0;             // voxel tables: 0 all row-major, 1 all tiled, 2 mixed
     cudaStream_t stream;
+    bool chained = true;        // see launch_chained
     // per-scene step limits and counters (device, n_scenes each); limits null:
     // no scene is frozen.  A frozen scene's particles keep their slots in the
     // sort, get no density task and are copied through by the force pass.
@@ -598,14 +622,35 @@ struct Launch {
     const int32_t* scene_step = nullptr;
 };
 
+// Launches a kernel of the step so that its grid is set up while the kernel
+// before it on the stream drains (programmatic dependent launch); captured into
+// a graph, the edge is programmatic too.  Every such kernel starts with
+// grid_wait (or grid_wait_index) in every thread, so a kernel's completion
+// implies the completion of all before it.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), int blocks, int threads, const Launch& L,
+                           A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = L.stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = L.chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // cell[s] = voxel id, or ~id (negative) for a particle in its scene's overflow
 // bucket; slot[s] = its arrival slot in the voxel.  Particles i0..i1 (i1 < 0:
 // all): the histogram may be filled in several launches over parts of the state
 // (the arrival order inside a voxel is dropped by the rank-gather).
 cudaError_t launch_hash_count(const Launch& L, const float4* pos, int32_t* cell, int32_t* slot,
                               int32_t* vcount, int i0 = 0, int i1 = -1);
+// status: scan_tiles(v_total) words, zero before the launch
 cudaError_t launch_scan(const Launch& L, const int32_t* vcount, int32_t* vstart,
-                        int32_t* tile_sums, int n_tiles);
+                        unsigned long long* status, int n_tiles);
 int scan_tiles(int v_total);
 cudaError_t launch_scatter(const Launch& L, const int32_t* cell, const int32_t* slot,
                            const int32_t* pid, const int32_t* vstart, const int32_t* vcount,
@@ -674,7 +719,8 @@ cudaError_t launch_integrate(const Launch& L, const float4* pos, const float4* v
                              const double* pos64, const int32_t* vstart, const int32_t* vcount,
                              const int32_t* scene_step, NbrList nbr, float4* pos_out,
                              float4* vel_out, int32_t* pid_out, double* pos64_out,
-                             float4* force_out, RareList rare = RareList{});
+                             float4* force_out, RareList rare = RareList{},
+                             int32_t* advance = nullptr);
 cudaError_t launch_integrate_range(const Launch& L, const float4* pos, const float4* vel,
                                    const float* rho, const float4* fin, const int32_t* pid,
                                    const double* pos64, const int32_t* vstart,

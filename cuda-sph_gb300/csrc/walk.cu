@@ -263,8 +263,8 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const int lane = threadIdx.x & 31;
     WcShared& S = sh[threadIdx.x >> 5];
     const unsigned lt = (1u << lane) - 1u;
-    const int n_tasks = *task_count;
-    if (task_offset) tasks += *task_offset;   // one bucket of a bucketed task list
+    const int n_tasks = *grid_wait(task_count);
+    if (task_offset) tasks += *after_wait(task_offset);   // one bucket of a bucketed task list
     // A warp's first task is its own number; each later one comes from a
     // counter (the cost of a task varies with its voxel's neighbourhood, and a
     // fixed share per warp left warps idle at the end of the pass, 15 % of its
@@ -274,7 +274,7 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     for (;;) {
         const int t = __shfl_sync(full, next, 0);    // uniform, also to the compiler
         if (t >= n_tasks) break;
-        const int2 task = tasks[t];
+        const int2 task = after_wait(tasks)[t];
         const int vid = task.x, d0 = task.y;
         const SceneDev& sc = scenes[scene_of_warp(d0, pbegin, n_scenes)];
         const int vst = __ldg(vstart + vid), vc = __ldg(vcount + vid);
@@ -715,11 +715,18 @@ k_integrate(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbe
             NbrList nbr, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
             int32_t* __restrict__ pid_out, double* __restrict__ pos64_out,
             float4* __restrict__ force_out, PidRange range, RareList rare,
-            const int32_t* __restrict__ step_limit) {
+            const int32_t* __restrict__ step_limit, int32_t* advance) {
     // kForceRare and kByList: a grid-stride loop over the deferred particles
     // or the listed slots; otherwise one particle per thread (the body runs once)
-    const int m_rare = kMode == kForceRare ? *rare.count : 0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x;; k += gridDim.x * blockDim.x) {
+    const int k_first = grid_wait((int)(blockIdx.x * blockDim.x + threadIdx.x));
+    const int m_rare = kMode == kForceRare ? *after_wait(rare.count) : 0;
+    // the last kernel of a step counts it, except in frozen scenes (the rare
+    // launch itself reads no counter)
+    if (kMode == kForceRare && advance) {
+        for (int i = k_first; i < n_scenes; i += gridDim.x * blockDim.x)
+            if (!(step_limit && advance[i] >= step_limit[i])) advance[i] += 1;
+    }
+    for (int k = k_first;; k += gridDim.x * blockDim.x) {
         // deferred particles are listed by row (kByRow) or by slot; rows_out:
         // the FP64 rows are written too
         constexpr bool by_row = kIdx == kByRow;
@@ -914,10 +921,9 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
                       : (L.layout == 1   ? k_density_wc<1, false>
                          : L.layout == 2 ? k_density_wc<2, false>
                                          : k_density_wc<0, false>);
-    kernel<<<blocks, kWcWarps * 32, 0, L.stream>>>(L.scenes, L.pbegin, L.n_scenes, L.n, pos, vel,
-                                                   vstart, vcount, rho, fin, nbr, tasks, task_count,
-                                                   task_next, task_offset, vrows);
-    return cudaGetLastError();
+    return launch_chained(kernel, blocks, kWcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
+                          L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, task_count, task_next,
+                          task_offset, vrows);
 }
 
 cudaError_t launch_gather_vel(const Launch& L, const int32_t* pid, const float4* vel_in,
@@ -969,35 +975,34 @@ cudaError_t launch_force_pass(const Launch& L, int m, const float4* pos, const f
                               const double* pos64, const int32_t* vstart, const int32_t* vcount,
                               const int32_t* scene_step, NbrList nbr, float4* pos_out,
                               float4* vel_out, int32_t* pid_out, double* pos64_out,
-                              float4* force_out, PidRange range, RareList rare) {
+                              float4* force_out, PidRange range, RareList rare,
+                              int32_t* advance) {
     // a slot list runs on a grid of at most 4 blocks per SM, each thread
     // taking list entries in turn: a bucket's list is a few waves long, and
     // no partial last wave is left
     const int grid = kIdx == kByList ? std::min(blocks_for(m), device_sm_count() * 4)
                                      : blocks_for(m);
-    if (L.pipe_scenes) {
-        k_integrate<true, kIdx, kForceAll><<<grid, kBlock, 0, L.stream>>>(
-            L.scenes, L.pbegin, L.n_scenes, L.n, L.pipe, pos, vel, rho, fin, pid, pos64, vstart,
-            vcount, scene_step, nbr, pos_out, vel_out, pid_out, pos64_out, force_out, range,
-            RareList{}, L.step_limit);
-    } else if (nbr.count && rare.count) {
-        k_integrate<false, kIdx, kForceLean><<<grid, kBlock, 0, L.stream>>>(
-            L.scenes, L.pbegin, L.n_scenes, L.n, L.pipe, pos, vel, rho, fin, pid, pos64, vstart,
-            vcount, scene_step, nbr, pos_out, vel_out, pid_out, pos64_out, force_out, range, rare,
-            L.step_limit);
-        const cudaError_t e = cudaGetLastError();
+    // Not chained to the density pass: started while density blocks still hold
+    // the SM's shared memory, the pass would keep the small L1 that leaves (28
+    // KB) to its end.  4,194,304 particles 0.45 ms, 0.75 chained; a 52k step 50
+    // and 64 us.
+    Launch Lf = L;
+    Lf.chained = false;
+    auto launch = [&](auto kernel, int blocks, RareList r, int32_t* adv) {
+        return launch_chained(kernel, blocks, kBlock, Lf, L.scenes, L.pbegin, L.n_scenes, L.n,
+                              L.pipe, pos, vel, rho, fin, pid, pos64, vstart, vcount, scene_step, nbr,
+                              pos_out, vel_out, pid_out, pos64_out, force_out, range, r, L.step_limit,
+                              adv);
+    };
+    if (L.pipe_scenes) return launch(k_integrate<true, kIdx, kForceAll>, grid, RareList{}, nullptr);
+    if (nbr.count && rare.count) {
+        const cudaError_t e = launch(k_integrate<false, kIdx, kForceLean>, grid, rare, nullptr);
         if (e != cudaSuccess) return e;
-        k_integrate<false, kIdx, kForceRare><<<device_sm_count(), kBlock, 0, L.stream>>>(
-            L.scenes, L.pbegin, L.n_scenes, L.n, L.pipe, pos, vel, rho, fin, pid, pos64, vstart,
-            vcount, scene_step, nbr, pos_out, vel_out, pid_out, pos64_out, force_out, range, rare,
-            L.step_limit);
-    } else {
-        k_integrate<false, kIdx, kForceAll><<<grid, kBlock, 0, L.stream>>>(
-            L.scenes, L.pbegin, L.n_scenes, L.n, L.pipe, pos, vel, rho, fin, pid, pos64, vstart,
-            vcount, scene_step, nbr, pos_out, vel_out, pid_out, pos64_out, force_out, range,
-            RareList{}, L.step_limit);
+        Lf.chained = L.chained;
+        return launch(k_integrate<false, kIdx, kForceRare>,
+                      std::min(blocks_for(std::max(m, L.n_scenes)), device_sm_count()), rare, advance);
     }
-    return cudaGetLastError();
+    return launch(k_integrate<false, kIdx, kForceAll>, grid, RareList{}, nullptr);
 }
 }  // namespace
 
@@ -1006,11 +1011,11 @@ cudaError_t launch_integrate(const Launch& L, const float4* pos, const float4* v
                              const double* pos64, const int32_t* vstart, const int32_t* vcount,
                              const int32_t* scene_step, NbrList nbr, float4* pos_out,
                              float4* vel_out, int32_t* pid_out, double* pos64_out,
-                             float4* force_out, RareList rare) {
+                             float4* force_out, RareList rare, int32_t* advance) {
     if (L.n == 0) return cudaSuccess;
     return launch_force_pass<kBySlot>(L, L.n, pos, vel, rho, fin, pid, pos64, vstart, vcount,
                                     scene_step, nbr, pos_out, vel_out, pid_out, pos64_out,
-                                    force_out, PidRange{}, rare);
+                                    force_out, PidRange{}, rare, advance);
 }
 
 cudaError_t launch_integrate_range(const Launch& L, const float4* pos, const float4* vel,
@@ -1027,10 +1032,10 @@ cudaError_t launch_integrate_range(const Launch& L, const float4* pos, const flo
     if (range.slots)
         return launch_force_pass<kByList>(L, m, pos, vel, rho, fin, pid, pos64, vstart, vcount,
                                           scene_step, nbr, pos_out, vel_out, pid_out, pos64_out,
-                                          nullptr, range, rare);
+                                          nullptr, range, rare, nullptr);
     return launch_force_pass<kByRow>(L, m, pos, vel, rho, fin, pid, pos64, vstart, vcount,
                                      scene_step, nbr, pos_out, vel_out, pid_out, pos64_out,
-                                     nullptr, range, rare);
+                                     nullptr, range, rare, nullptr);
 }
 
 cudaError_t launch_neighbours(const Launch& L, const float4* pos, const int32_t* vstart,
