@@ -509,17 +509,19 @@ struct Acc {
     }
 };
 
-// Two of those sums in one register pair, with sm_100's packed FP32 adds:
-// each element is rounded exactly as the scalar add rounds it, so the x and
-// y components give the scalar Acc's bits with half the add instructions.
+// Two of those sums in one register pair, with sm_100's packed FP32 arithmetic
+// (half the instructions of two scalar sums).  A term m x enters fused, y =
+// m x - c in one rounding; written out, since the compiler fuses a packed
+// product with a packed sum by itself, and the other passes over the same terms
+// (k_integrate_group) have to round alike.
 template <bool kPlain>
 struct Acc2 {
     float2 s = make_float2(0.0f, 0.0f), c = make_float2(0.0f, 0.0f);
-    __device__ __forceinline__ void add(float2 x) {
+    __device__ __forceinline__ void add(float2 m, float2 x) {
         if (kPlain) {
-            s = __fadd2_rn(s, x);
+            s = __ffma2_rn(m, x, s);
         } else {
-            const float2 y = __fadd2_rn(x, make_float2(-c.x, -c.y));
+            const float2 y = __ffma2_rn(m, x, make_float2(-c.x, -c.y));
             const float2 t = __fadd2_rn(s, y);
             c = __fadd2_rn(__fadd2_rn(t, make_float2(-s.x, -s.y)), make_float2(-y.x, -y.y));
             s = t;
@@ -552,11 +554,11 @@ __device__ __forceinline__ void add_pair(ForceSums<kPlain>& f, const float4& vi,
     const float inv_r = 1.0f / r;
     const float t = __fmaf_rn(-r, inv_h, 1.0f);
     const float g = ((a_i + aj.x) * gw) * (t * t) * inv_r;
-    f.pxy.add(__fmul2_rn(make_float2(g, g), dxy));
+    f.pxy.add(make_float2(g, g), dxy);
     f.pz.add(g * dz);
     const float l = (lw * t) * aj.y;
     const float2 dv = __fadd2_rn(make_float2(vj.x, vj.y), make_float2(-vi.x, -vi.y));
-    f.vxy.add(__fmul2_rn(make_float2(l, l), dv));
+    f.vxy.add(make_float2(l, l), dv);
     f.vz.add(l * (vj.z - vi.z));
 }
 
@@ -864,6 +866,134 @@ k_integrate(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbe
     }
 }
 
+// The list pass of small scenes (kForceLean's work and results, box scenes, by
+// slot): eight lanes per particle.  Thread per particle, such a pass is one
+// thread's chain of loads and sums long, with most of the chip idle.  Here each
+// lane computes the terms of four list entries, and six lanes then add up one
+// component each, in list order with the same compensated sums: the same bits.
+// 145 warp instructions per particle instead of 80, but a chain of one load and
+// one sum over 32 entries; see kGroupParticles for where the lines cross.
+constexpr int kGroupLanes = 8;
+constexpr int kGroupsPerBlock = kBlock / kGroupLanes;
+// Up to this many particles the step takes this pass.  Whole steps, with it and
+// with a thread per particle: 1,024 particles 24.6 and 30.2 us, 8,192 27.2 and
+// 33.0, 17,280 35.2 and 36.8, 33,600 43.1 and 39.5.
+constexpr int kGroupParticles = 20000;
+static_assert(kListCap == 4 * kGroupLanes, "four list entries per lane");
+
+__global__ void __launch_bounds__(kBlock)
+k_integrate_group(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
+                  int n_scenes, int n, const float4* __restrict__ pos,
+                  const float4* __restrict__ vel, const float* __restrict__ rho,
+                  const float4* __restrict__ fin, const int32_t* __restrict__ pid, NbrList nbr,
+                  float4* __restrict__ pos_out, float4* __restrict__ vel_out,
+                  int32_t* __restrict__ pid_out, RareList rare,
+                  const int32_t* __restrict__ step_limit, const int32_t* __restrict__ scene_step) {
+    // by particle and list entry: the terms as Acc2 and Acc take them, that is
+    // factor and difference of the x and y components, product of the z ones:
+    // g, dx, dy, g dz, then the same of the viscosity
+    __shared__ float terms[kGroupsPerBlock][8][kListCap + 1];
+    const int tid = grid_wait((int)threadIdx.x);
+    const int sub = tid % kGroupLanes, g = tid / kGroupLanes;
+    const unsigned mine = ((1u << kGroupLanes) - 1u) << (tid & 31 & ~(kGroupLanes - 1));
+    const int s = blockIdx.x * kGroupsPerBlock + g;
+    if (s >= n) return;                      // whole groups
+    const int si = scene_of(s, pbegin, n_scenes);
+    const SceneDev& sc = scenes[si];
+    if (scene_frozen(step_limit, scene_step, si)) {
+        if (sub == 0) {
+            pos_out[s] = __ldg(pos + s);
+            vel_out[s] = __ldg(vel + s);
+            pid_out[s] = __ldg(pid + s);
+        }
+        return;
+    }
+    const int cnt = __ldg(nbr.count + s);
+    const int4 row = __ldg(reinterpret_cast<const int4*>(nbr.idx + (size_t)s * kListCap) + sub);
+    float4 fa, fb;
+    ldg256(fin + 2 * s, fa, fb);
+    const float rho_i = __ldg(rho + s);
+    const int p_id = __ldg(pid + s);
+    const float2 ai = make_float2(fa.w, fb.w);
+    const float inv_h = 1.0f / sc.h;
+    const float gw = sc.grad_w_const, lw = sc.lap_w_const;
+    const int js[4] = {row.x, row.y, row.z, row.w};
+    float4 pq[4], vq[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)              // past the end of the list: the particle itself
+        ldg256(fin + 2 * (4 * sub + e < cnt ? js[e] : s), pq[e], vq[e]);
+    bool bad = false;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int k = 4 * sub + e;
+        if (k < cnt) {
+            // the terms of add_pair, before they are added
+            const float2 aj = make_float2(pq[e].w, vq[e].w);
+            bad |= !(fabsf(aj.x * aj.y) < INFINITY);
+            const float dx = __fsub_rn(fa.x, pq[e].x), dy = __fsub_rn(fa.y, pq[e].y),
+                        dz = __fsub_rn(fa.z, pq[e].z);
+            float d2 = __fmul_rn(dx, dx);
+            d2 = __fmaf_rn(dy, dy, d2);
+            d2 = __fmaf_rn(dz, dz, d2);
+            const float r = sqrtf(d2);
+            const float inv_r = 1.0f / r;
+            const float t = __fmaf_rn(-r, inv_h, 1.0f);
+            const float gr = ((ai.x + aj.x) * gw) * (t * t) * inv_r;
+            const float l = (lw * t) * aj.y;
+            float* T = &terms[g][0][k];
+            constexpr int N = kListCap + 1;
+            T[0] = gr;
+            T[N] = dx;
+            T[2 * N] = dy;
+            T[3 * N] = __fmul_rn(gr, dz);
+            T[4 * N] = l;
+            T[5 * N] = __fsub_rn(vq[e].x, fb.x);
+            T[6 * N] = __fsub_rn(vq[e].y, fb.y);
+            T[7 * N] = __fmul_rn(l, __fsub_rn(vq[e].z, fb.z));
+        }
+    }
+    const bool ok = cnt >= 0 && fabsf(ai.x * ai.y) < INFINITY && !__any_sync(mine, bad);
+    if (!ok) {                               // the same in every lane of the group
+        if (sub == 0) rare.idx[rare.base + atomicAdd(rare.count, 1)] = s;
+        return;
+    }
+    __syncwarp(mine);
+    // lanes 0 to 2: pressure x, y, z; 3 to 5: viscosity
+    float sum = 0.0f, c = 0.0f;
+    if (sub < 6) {
+        const bool z = sub == 2 || sub == 5;
+        const float* m = terms[g][sub < 3 ? 0 : 4];
+        const float* x = terms[g][(sub < 3 ? 1 : 2) + sub];
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) {
+            const float y = __fmaf_rn(z ? 1.0f : m[k], x[k], -c);
+            const float t = __fadd_rn(sum, y);
+            c = __fsub_rn(__fsub_rn(t, sum), y);
+            sum = t;
+        }
+    }
+    const float visc = __shfl_down_sync(mine, sum, 3, kGroupLanes);
+    // lane a < 3: component a of the integration and the wall response
+    const int a = sub < 3 ? sub : 0;
+    const float vscale = sc.mass * sc.visc * ai.y;
+    const float F = (sc.ext[a] + -sum) + clamp1(cnt ? visc * vscale : 0.0f);
+    float v = a == 0 ? fb.x : a == 1 ? fb.y : fb.z;
+    v = v + (F / rho_i) * sc.dt;
+    float x = a == 0 ? fa.x : a == 1 ? fa.y : fa.z;
+    x = x + v * sc.dt;
+    bool bounced = false;
+    if (x < 0.0f) { x = sc.wall_lo; bounced = true; }
+    if (x > sc.space[a]) { x = sc.wall_hi[a]; bounced = true; }
+    if (bounced) v = -v * sc.damp;
+    const float x1 = __shfl_down_sync(mine, x, 1, kGroupLanes), x2 = __shfl_down_sync(mine, x, 2, kGroupLanes);
+    const float v1 = __shfl_down_sync(mine, v, 1, kGroupLanes), v2 = __shfl_down_sync(mine, v, 2, kGroupLanes);
+    if (sub == 0) {
+        pos_out[s] = make_float4(x, x1, x2, 0.0f);
+        vel_out[s] = make_float4(v, v1, v2, 0.0f);
+        pid_out[s] = p_id;
+    }
+}
+
 __global__ void __launch_bounds__(kBlock)
 k_neighbours(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
              int n_scenes, int n, const float4* __restrict__ pos,
@@ -996,7 +1126,12 @@ cudaError_t launch_force_pass(const Launch& L, int m, const float4* pos, const f
     };
     if (L.pipe_scenes) return launch(k_integrate<true, kIdx, kForceAll>, grid, RareList{}, nullptr);
     if (nbr.count && rare.count) {
-        const cudaError_t e = launch(k_integrate<false, kIdx, kForceLean>, grid, rare, nullptr);
+        const cudaError_t e =
+            kIdx == kBySlot && !force_out && m <= kGroupParticles
+                ? launch_chained(k_integrate_group, (m + kGroupsPerBlock - 1) / kGroupsPerBlock, kBlock,
+                                 Lf, L.scenes, L.pbegin, L.n_scenes, L.n, pos, vel, rho, fin, pid, nbr,
+                                 pos_out, vel_out, pid_out, rare, L.step_limit, scene_step)
+                : launch(k_integrate<false, kIdx, kForceLean>, grid, rare, nullptr);
         if (e != cudaSuccess) return e;
         Lf.chained = L.chained;
         return launch(k_integrate<false, kIdx, kForceRare>,
