@@ -99,7 +99,12 @@ constexpr int kHostEvents = kHostOrganizedEvent + 1;
 constexpr int kTcCounter = 4 + (kHostRanges > kPipeRanges ? kHostRanges : kPipeRanges);
 constexpr int kCounters = kTcCounter + 2;
 constexpr size_t kCountersPad = 64;      // ints; what follows stays 128-byte aligned
-static_assert(kCounters <= (int)kCountersPad, "counters");
+constexpr int kOverCounter = (int)kCountersPad - 2;   // 64-bit: units of the list pool taken
+static_assert(kCounters <= kOverCounter, "counters");
+// pool of the lists that do not fit their rows (scenes without a cap): 128
+// entries per particle, 8 GB at most
+constexpr size_t kOverPerParticle = 128 / 8;
+constexpr size_t kOverMax = (size_t)1 << 28;
 // contexts of sparse and dense scenes: voxels of at most this many particles go
 // to k_density_tc, the others to k_density_wc
 constexpr int kTcVoxel = 48;
@@ -143,6 +148,8 @@ struct SphgbCtx {
     int32_t* big_list = nullptr;     // voxels with more than kBigVoxel members
     int32_t* big_count = nullptr;     // counters: [0] big voxels, [1] density tasks, [2] tasks taken,
                                       // [3 + r] deferred particles of force pass r (kCounters)
+    int32_t* over = nullptr;          // pool of long neighbour lists (NbrList), may be missing
+    unsigned long long over_units = 0;
     int32_t* rare = nullptr;          // deferred particles of the force pass (RareList)
     int2* tasks = nullptr;             // (voxel, first slot) per run of <= kTaskRun slots
     // the neighbour rows in nbr, pidB and posB are those of the latest step
@@ -181,7 +188,7 @@ struct SphgbCtx {
         size_t scenes = 0, scenes_ref = 0, pbegin = 0, pipe = 0, cell = 0, slot_of = 0, slot = 0, tmp_pid = 0,
                vstart = 0,
                counts = 0, posB = 0, velB = 0, pidB = 0, fin = 0, big_list = 0,
-               rare = 0, tasks = 0, nbr_idx = 0, nbr_count = 0, pos64B = 0, chunks = 0,
+               over = 0, rare = 0, tasks = 0, nbr_idx = 0, nbr_count = 0, pos64B = 0, chunks = 0,
                partials = 0;
     } cap;
     // tuning (sphgb_ctx_set_tuning)
@@ -225,6 +232,16 @@ struct SphgbCtx {
     DensityPass density_pass() const {
         if (layout == 1 || uncapped) return kPassTc;
         return layout == 2 ? kPassBoth : kPassWc;
+    }
+    // the step's neighbour lists: with the pool when k_density_tc writes them all
+    NbrList step_nbr() const {
+        NbrList l = nbr;
+        if (uncapped && over && density_variant == SPHGB_DENSITY_WARP) {
+            l.over = over;
+            l.over_used = reinterpret_cast<unsigned long long*>(counts + kOverCounter);
+            l.over_units = over_units;
+        }
+        return l;
     }
     TaskLists task_lists() const {
         TaskLists t;
@@ -279,7 +296,7 @@ void free_ctx(SphgbCtx* c) {
     void* ptrs[] = {c->d_scenes, c->d_scenes_ref, c->d_pbegin, c->d_pipe, c->cell, c->slot_of, c->slot, c->tmp_pid,
                     c->vstart, c->counts, c->posB, c->velB, c->pidB,
                     c->pos64B, c->fin, c->owned, c->stage, c->d_chunks, c->d_partials,
-                    c->big_list, c->rare, c->nbr.idx, c->nbr.count, c->tasks,
+                    c->big_list, c->over, c->rare, c->nbr.idx, c->nbr.count, c->tasks,
                     c->d_check};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -768,11 +785,11 @@ int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int rang
     rare.base = !range ? 0 : range->slots ? (int)(range->slots - c->slots_b) : range->i0;
     if (range)
         SPHGB_CUDA(launch_integrate_range(L, c->posB, c->velB, c->rho, c->fin, c->pidB, p64B,
-                                          c->vstart, c->vcount, c->scene_step, c->nbr, pos_o,
+                                          c->vstart, c->vcount, c->scene_step, c->step_nbr(), pos_o,
                                           vel_o, pid_o, p64_o, *range, rare));
     else
         SPHGB_CUDA(launch_integrate(L, c->posB, c->velB, c->rho, c->fin, c->pidB, p64B, c->vstart,
-                                    c->vcount, c->scene_step, c->nbr, pos_o, vel_o, pid_o, p64_o,
+                                    c->vcount, c->scene_step, c->step_nbr(), pos_o, vel_o, pid_o, p64_o,
                                     nullptr, rare, advance ? c->scene_step : nullptr));
     return SPHGB_OK;
 }
@@ -818,21 +835,23 @@ int enqueue_step(SphgbCtx* c, cudaStream_t st, cudaEvent_t* ev = nullptr,
                               p64B, c->vstart, c->vcount, ev ? ev + 1 : nullptr, lists, hashed);
     if (rc) return rc;
     if (organized) SPHGB_CUDA(cudaEventRecord(organized, st));
+    const NbrList nbr = c->step_nbr();
     if (warp) {
         const SphgbCtx::DensityPass pass = c->density_pass();
         if (pass == SphgbCtx::kPassTc)
             SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                         c->nbr, lists.list, 1, lists.count, c->big_count + 2));
+                                         nbr, lists.list, 1, lists.count, c->big_count + 2,
+                                         c->uncapped));
         else
             SPHGB_CUDA(launch_density_wc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                         c->nbr, lists.list, lists.count, c->big_count + 2));
+                                         nbr, lists.list, lists.count, c->big_count + 2));
         if (pass == SphgbCtx::kPassBoth)
             SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                         c->nbr, lists.tc_last, -1, lists.tc_count,
-                                         lists.tc_count + 1));
+                                         nbr, lists.tc_last, -1, lists.tc_count,
+                                         lists.tc_count + 1, false));
     } else
         SPHGB_CUDA(launch_density(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                  c->nbr));
+                                  nbr));
     if (ev) SPHGB_CUDA(cudaEventRecord(ev[5], st));
     if (density_done) SPHGB_CUDA(cudaEventRecord(density_done, st));
     if (vel_ready) {
@@ -964,6 +983,11 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
     c->any_pipe = any_pipe;
     c->uncapped = false;
     for (const SceneDev& d : c->h_scenes) c->uncapped |= d.cap > kListCap;
+    if (c->uncapped && N > 0) {
+        c->over_units = std::min(N * kOverPerParticle, kOverMax);
+        // without the pool the force pass walks again: slower, the same results
+        if (ensure(&c->over, k.over, 8 * (size_t)c->over_units) != SPHGB_OK) g_last_error.clear();
+    }
     // the caller binds (new) state and outputs for the new layout
     c->bound = false;
     c->nbr_valid = false;

@@ -330,13 +330,14 @@ __device__ __forceinline__ uint32_t drop_first(uint32_t w, int d) {
 
 // Phase 2 for one lane: visits the next n accepted candidates of its home,
 // adds their density terms and stores their slots from shared-memory address
-// `row` on (kBound: below row_end only), passing over the one at address
-// `self`; returns where the row ends.  The words hold at least n more bits: n
-// counts bits of theirs.  A lane that meets an empty word lets a turn pass.
+// `row` on (kBound: below row_end only, and into `over` from `row` on when
+// given), passing over the one at address `self`; returns where the row ends.
+// The words hold at least n more bits: n counts bits of theirs.  A lane that
+// meets an empty word lets a turn pass.
 template <bool kBound>
 __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uint32_t row_end,
                                            uint32_t self, const float4& pi, float inv_h2,
-                                           Kahan& acc) {
+                                           Kahan& acc, int32_t* over = nullptr) {
     while (n > 0) {
         C.advance_if_empty();
         // place of the first bit; -1 in an empty word, which is never the
@@ -360,6 +361,7 @@ __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uin
             acc = a;
             if (!kBound || row < row_end)
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(row), "f"(pj.w) : "memory");
+            if (kBound && over) *over++ = __float_as_int(pj.w);
             row += 4;
         }
     }
@@ -367,8 +369,8 @@ __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uin
 }
 
 // kLayout: 0 every scene's voxel table row-major, 1 every one tiled, 2 per scene.
-// Task t is at tasks[t * dir].
-template <int kLayout>
+// Task t is at tasks[t * dir].  kUncapped: some scene's cap is beyond kListCap.
+template <int kLayout, bool kUncapped>
 __global__ void __launch_bounds__(kTcWarps * 32, 6)
 k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
              int n_scenes, int n, const float4* __restrict__ pos,
@@ -496,17 +498,36 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         // that no home can reach are passed over.
         const bool cull = !sc.walk_trunc && M > kTcCullMin;
         const unsigned reach = cull ? reach_mask(pi, vx, vy, vz, sc) : 0u;
-        const bool uncapped = cap > kListCap;   // the row may not hold every neighbour
+        // the row may not hold every neighbour
+        const bool uncapped = kUncapped && cap > kListCap;
         const float inv_h2 = sc.inv_h2;
         int cnt = 0;       // home ih: accepted candidates so far (self included)
         int others = 0;    // of those, not the particle itself
         Kahan acc;         // lane i: entries of home i below kSumSplit, lane 16 + i: the rest
         Kahan first;       // uncapped: the first part; acc of lane i then sums every entry
+        long long unit = -1;     // uncapped: the home's place in the pool
         for (int c0 = 0; c0 < M; c0 += kTcChunk) {
             const int c1 = min(M, c0 + kTcChunk);
             int T, gh, Th;
             const int G = tc_decide(S, T, gh, Th, cnt, c_t, cap, c0, c1, Pk, ck, nzk, cull, reach, A, Cq, ballots, F, pi,
                                     pos, n, sc);
+            if (uncapped && c0 == 0 && nbr.over) {
+                // room for the lists that will not fit their rows: of known
+                // length when this chunk is the walk, else as long as the walk
+                const int most = c1 == M ? T : M;
+                const int need = home && most > kListCap ? (most + 7) >> 3 : 0;
+                int incl = need;
+#pragma unroll
+                for (int o = 1; o < kTaskRun; o <<= 1) {
+                    const int v = __shfl_up_sync(full, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int total = __shfl_sync(full, incl, kTaskRun - 1);
+                unsigned long long u = 0;
+                if (lane == 0 && total) u = atomicAdd(nbr.over_used, (unsigned long long)total);
+                u = __shfl_sync(full, u, 0);
+                if (u + total <= nbr.over_units) unit = need ? (long long)u + incl - need : -1;
+            }
             const int n_all = ih < c_t ? max(min(T, cap - cnt), 0) : 0;   // entries used here
             int n_lo = min(n_all, max(kSumSplit - cnt, 0)), n_hi = n_all - n_lo;
             // where the lane starts: the lower one at the first word, the upper
@@ -528,10 +549,13 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             if (!uncapped) {
                 end = tc_sum<false>(C, upper ? n_hi : n_lo, row, 0u, self, pi, inv_h2, acc);
             } else {
-                const uint32_t row_end = row0 + 4 * kListCap;
-                end = tc_sum<true>(C, upper ? n_hi : n_lo, row, row_end, self, pi, inv_h2, acc);
+                // the lower lane goes over every entry and lists them
+                const uint32_t row_end = upper ? row0 : row0 + 4 * kListCap;
+                int32_t* over = unit >= 0 ? nbr.over + 8 * unit + others : nullptr;    // lower lanes
+                end = tc_sum<true>(C, upper ? n_hi : n_lo, row, row_end, self, pi, inv_h2, acc, over);
                 if (cnt < kSumSplit) first = acc;
-                end = tc_sum<true>(C, upper ? 0 : n_hi, end, row_end, self, pi, inv_h2, acc);
+                if (over) over += (end - row) >> 2;
+                end = tc_sum<true>(C, upper ? 0 : n_hi, end, row_end, self, pi, inv_h2, acc, over);
             }
             // entries of both lanes (uncapped: the lower lane went over all)
             const int mine = (int)(end - row) >> 2;
@@ -542,6 +566,11 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             if (!__any_sync(full, home && cnt < cap)) break;
         }
         __syncwarp();
+        if (kUncapped && home && others > kListCap) {
+            S.list[ih][0] = unit >= 0 ? others : 0;
+            S.list[ih][1] = (int)unit;
+        }
+        if (kUncapped) __syncwarp();
         // list rows, four homes at a time, 16 bytes per lane (entries past a
         // row's count are not read by anyone)
         if (nbr.idx) {
@@ -579,13 +608,18 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
 cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
                               float4* fin, NbrList nbr, const int2* tasks, int dir,
-                              const int32_t* task_count, int32_t* task_next) {
+                              const int32_t* task_count, int32_t* task_next, bool uncapped) {
     if (L.n == 0) return cudaSuccess;
     // persistent grid: up to 6 blocks of 4 warps per SM (shared memory), warps
     // take tasks in turn; small scenes get about a warp per task, so that the
     // tasks spread over the SMs (a task's latency is most of their pass)
     const int blocks = std::min((L.n + 8 * kTcWarps - 1) / (8 * kTcWarps), device_sm_count() * 6);
-    auto kernel = L.layout == 1 ? k_density_tc<1> : L.layout == 2 ? k_density_tc<2> : k_density_tc<0>;
+    auto kernel = uncapped ? (L.layout == 1   ? k_density_tc<1, true>
+                              : L.layout == 2 ? k_density_tc<2, true>
+                                              : k_density_tc<0, true>)
+                           : (L.layout == 1   ? k_density_tc<1, false>
+                              : L.layout == 2 ? k_density_tc<2, false>
+                                              : k_density_tc<0, false>);
     return launch_chained(kernel, blocks, kTcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
                           L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, dir, task_count,
                           task_next);

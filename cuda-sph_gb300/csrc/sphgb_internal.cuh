@@ -558,7 +558,28 @@ constexpr int kListCap = 32;
 struct NbrList {
     int32_t* idx = nullptr;     // kListCap * n entries
     int32_t* count = nullptr;   // n entries; -1 = more than kListCap neighbours
+    // contexts with scenes without a cap: the lists of the particles of count
+    // -1, in units of 8 entries taken from one pool; such a particle's row
+    // starts with {its number of neighbours, first unit}, {0, -} when the pool
+    // had no room.  over null: rows of count -1 hold nothing.  Without the pool
+    // the force pass walked again, one thread per particle: 32,768 particles
+    // with 47 neighbours 190 -> 23 us.
+    int32_t* over = nullptr;
+    unsigned long long* over_used = nullptr;    // units taken, zero before the density pass
+    unsigned long long over_units = 0;
 };
+// the list of a particle: its row, or its place in the pool; cnt -1: none
+__device__ __forceinline__ const int32_t* nbr_row(const NbrList& nbr, int s, int& cnt) {
+    const int32_t* row = nbr.idx ? nbr.idx + (size_t)s * kListCap : nullptr;
+    if (cnt < 0 && nbr.over) {
+        const int2 e = __ldg(reinterpret_cast<const int2*>(row));
+        if (e.x > 0) {
+            cnt = e.x;
+            row = nbr.over + 8 * (size_t)(unsigned)e.y;
+        }
+    }
+    return row;
+}
 
 // Force pass over a range of particles in original order (scene offset +
 // particle id): particle i is at slot slot_of[i], and its next position and
@@ -698,11 +719,12 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
                               float4* fin, NbrList nbr, const int2* tasks,
                               const int32_t* task_count, int32_t* task_next,
                               const int32_t* task_offset = nullptr, VelRows vrows = VelRows{});
-// the same on the tensor cores; task t is at tasks[t * dir]
+// the same on the tensor cores; task t is at tasks[t * dir]; uncapped: some
+// scene's cap is beyond kListCap
 cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
                               float4* fin, NbrList nbr, const int2* tasks, int dir,
-                              const int32_t* task_count, int32_t* task_next);
+                              const int32_t* task_count, int32_t* task_next, bool uncapped);
 // k_gather_vel over the slots of a bucket of density tasks
 cudaError_t launch_gather_vel_tasks(const Launch& L, const int32_t* pid, const int2* tasks,
                                     const int32_t* task_count, const int32_t* task_offset,

@@ -786,8 +786,8 @@ k_integrate(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbe
         const float4 vi = make_float4(fb.x, fb.y, fb.z, 0.0f);
         const float2 ai = make_float2(fa.w, fb.w);
         const float rho_i = __ldg(rho + s);
-        const int cnt = nbr.count ? __ldg(nbr.count + s) : -1;
-        const int32_t* list = nbr.idx ? nbr.idx + (size_t)s * kListCap : nullptr;
+        int cnt = nbr.count ? __ldg(nbr.count + s) : -1;
+        const int32_t* list = nbr_row(nbr, s, cnt);
         Forces f;
         if (kMode == kForceLean) {
             ForceSums<false> fs;
@@ -1127,7 +1127,7 @@ cudaError_t launch_force_pass(const Launch& L, int m, const float4* pos, const f
     if (L.pipe_scenes) return launch(k_integrate<true, kIdx, kForceAll>, grid, RareList{}, nullptr);
     if (nbr.count && rare.count) {
         const cudaError_t e =
-            kIdx == kBySlot && !force_out && m <= kGroupParticles
+            kIdx == kBySlot && !force_out && m <= kGroupParticles && !nbr.over
                 ? launch_chained(k_integrate_group, (m + kGroupsPerBlock - 1) / kGroupsPerBlock, kBlock,
                                  Lf, L.scenes, L.pbegin, L.n_scenes, L.n, pos, vel, rho, fin, pid, nbr,
                                  pos_out, vel_out, pid_out, rare, L.step_limit, scene_step)
