@@ -417,28 +417,49 @@ int build_scene(const SphgbSceneParams& p, int n_pipe_rows_total, SceneDev& d,
     return SPHGB_OK;
 }
 
+// Rows of 3 doubles go through shared memory, so that a warp's accesses are
+// whole lines: they may go over the host link (host_entry's direct order), and
+// on the device a thread's own 24 bytes touch three times the sectors.
+__device__ __forceinline__ void load_rows(double* buf, const double* __restrict__ src, int i, int m) {
+    for (int k = threadIdx.x; k < 3 * m; k += kBlock) buf[k] = src[3 * (size_t)i + k];
+}
+__device__ __forceinline__ void store_rows(double* __restrict__ dst, const double* buf, int i, int m) {
+    for (int k = threadIdx.x; k < 3 * m; k += kBlock) dst[3 * (size_t)i + k] = buf[k];
+}
+
 // rows i0..n-1 of an FP64 AoS state into the float4 state (and the pipe
-// accumulator); vel or pos may be null
-__global__ void k_load_aos(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
-                           int n_scenes, int i0, int n, const double* __restrict__ pos,
-                           const double* __restrict__ vel, float4* __restrict__ pos_out,
-                           float4* __restrict__ vel_out, int32_t* __restrict__ pid_out,
-                           double* __restrict__ pos64_out) {
-    const int i = i0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (vel)
-        vel_out[i] = make_float4((float)vel[3 * i], (float)vel[3 * i + 1], (float)vel[3 * i + 2], 0.0f);
-    if (!pos) return;   // velocities only
-    const int si = scene_of(i, pbegin, n_scenes);
-    const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
-    pos_out[i] = make_float4((float)x, (float)y, (float)z, 0.0f);
-    pid_out[i] = i - __ldg(pbegin + si);
-    if (pos64_out) {
-        // the FP64 accumulator takes the input as given (an exported pipe state
-        // reloads bit-exactly); FP32-representable input makes it equal pos
-        pos64_out[3 * i] = x;
-        pos64_out[3 * i + 1] = y;
-        pos64_out[3 * i + 2] = z;
+// accumulator); vel or pos may be null.  kHost: rows in host memory, through
+// shared memory.
+template <bool kHost>
+__global__ void __launch_bounds__(kBlock)
+k_load_aos(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
+           int n_scenes, int i0, int n, const double* __restrict__ pos,
+           const double* __restrict__ vel, float4* __restrict__ pos_out,
+           float4* __restrict__ vel_out, int32_t* __restrict__ pid_out,
+           double* __restrict__ pos64_out) {
+    __shared__ double buf[kHost ? 6 * kBlock : 1];
+    const int first = i0 + blockIdx.x * kBlock;
+    const int m = min(kBlock, n - first), t = threadIdx.x;
+    const double *ps = pos + 3 * (size_t)first, *vs = vel + 3 * (size_t)first;
+    if (kHost) {
+        if (pos) load_rows(buf, pos, first, m);
+        if (vel) load_rows(buf + 3 * kBlock, vel, first, m);
+        __syncthreads();
+        ps = buf;
+        vs = buf + 3 * kBlock;
+    }
+    const int i = first + t;
+    if (t < m) {
+        if (vel)
+            vel_out[i] = make_float4((float)vs[3 * t], (float)vs[3 * t + 1], (float)vs[3 * t + 2], 0.0f);
+        if (pos) {
+            pos_out[i] = make_float4((float)ps[3 * t], (float)ps[3 * t + 1], (float)ps[3 * t + 2], 0.0f);
+            pid_out[i] = i - __ldg(pbegin + scene_of(i, pbegin, n_scenes));
+            // the FP64 accumulator takes the input as given (an exported pipe state
+            // reloads bit-exactly); FP32-representable input makes it equal pos
+            if (pos64_out)
+                for (int a = 0; a < 3; ++a) pos64_out[3 * (size_t)i + a] = ps[3 * t + a];
+        }
     }
     (void)scenes;
 }
@@ -451,37 +472,42 @@ __global__ void k_slot_of(const int32_t* __restrict__ pbegin, int n_scenes, int 
     slot_of[__ldg(pbegin + scene_of(s, pbegin, n_scenes)) + pid[s]] = s;
 }
 
-// state in original particle order as FP64 AoS: one thread per output row,
-// so the writes are coalesced (they may go to mapped host memory)
-__global__ void k_store_aos(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
-                            int n_scenes, int n, const float4* __restrict__ pos,
-                            const float4* __restrict__ vel, const float* __restrict__ rho,
-                            const int32_t* __restrict__ slot_of, const double* __restrict__ pos64,
-                            double* __restrict__ pos_out, double* __restrict__ vel_out,
-                            double* __restrict__ rho_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int si = scene_of(i, pbegin, n_scenes);
-    const int s = __ldg(slot_of + i);
-    if (pos_out) {
-        if (pos64 && scenes[si].mode == 1) {
-            pos_out[3 * i] = pos64[3 * s];
-            pos_out[3 * i + 1] = pos64[3 * s + 1];
-            pos_out[3 * i + 2] = pos64[3 * s + 2];
-        } else {
-            const float4 p = pos[s];
-            pos_out[3 * i] = p.x;
-            pos_out[3 * i + 1] = p.y;
-            pos_out[3 * i + 2] = p.z;
+// state in original particle order as FP64 AoS: one thread per output row (the
+// rows may be in host memory)
+__global__ void __launch_bounds__(kBlock)
+k_store_aos(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
+            int n_scenes, int n, const float4* __restrict__ pos,
+            const float4* __restrict__ vel, const float* __restrict__ rho,
+            const int32_t* __restrict__ slot_of, const double* __restrict__ pos64,
+            double* __restrict__ pos_out, double* __restrict__ vel_out,
+            double* __restrict__ rho_out) {
+    __shared__ double ps[3 * kBlock], vs[3 * kBlock];
+    const int first = blockIdx.x * kBlock;
+    const int m = min(kBlock, n - first), t = threadIdx.x;
+    if (t < m) {
+        const int i = first + t;
+        const int s = __ldg(slot_of + i);
+        if (pos_out) {
+            if (pos64 && scenes[scene_of(i, pbegin, n_scenes)].mode == 1) {
+                for (int a = 0; a < 3; ++a) ps[3 * t + a] = pos64[3 * (size_t)s + a];
+            } else {
+                const float4 p = pos[s];
+                ps[3 * t] = p.x;
+                ps[3 * t + 1] = p.y;
+                ps[3 * t + 2] = p.z;
+            }
         }
+        if (vel_out) {
+            const float4 v = vel[s];
+            vs[3 * t] = v.x;
+            vs[3 * t + 1] = v.y;
+            vs[3 * t + 2] = v.z;
+        }
+        if (rho_out) rho_out[i] = rho ? (double)rho[s] : 0.0;
     }
-    if (vel_out) {
-        const float4 v = vel[s];
-        vel_out[3 * i] = v.x;
-        vel_out[3 * i + 1] = v.y;
-        vel_out[3 * i + 2] = v.z;
-    }
-    if (rho_out) rho_out[i] = rho ? (double)rho[s] : 0.0;
+    __syncthreads();
+    if (pos_out) store_rows(pos_out, ps, first, m);
+    if (vel_out) store_rows(vel_out, vs, first, m);
 }
 
 __global__ void k_step_counter(int32_t* scene_step, int n_scenes, const int32_t* step_limit) {
@@ -1145,7 +1171,7 @@ int sphgb_ctx_load_aos_f64(SphgbCtx* ctx, const double* d_pos_aos, const double*
     if (ctx->n == 0) return SPHGB_OK;
     if (!d_pos_aos || !d_vel_aos) return fail(SPHGB_ERR_INVALID, "null input");
     cudaStream_t st = as_stream(stream);
-    k_load_aos<<<blocks(ctx->n), kBlock, 0, st>>>(ctx->d_scenes, ctx->d_pbegin, ctx->n_scenes,
+    k_load_aos<false><<<blocks(ctx->n), kBlock, 0, st>>>(ctx->d_scenes, ctx->d_pbegin, ctx->n_scenes,
                                                  0, ctx->n, d_pos_aos, d_vel_aos, ctx->posA,
                                                  ctx->velA, ctx->pidA, ctx->pos64A);
     SPHGB_CUDA(cudaGetLastError());
@@ -1655,6 +1681,63 @@ int host_order_for_call(const SphgbCtx* c) {
 }
 }  // namespace
 
+extern "C++" {
+namespace {
+// whether kernels reach every host page through the host's own page tables
+bool pageable_access() {
+    static std::atomic<int> cache[64] = {};      // 1: no, 2: yes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int v = cache[dev].load(std::memory_order_relaxed);
+    if (!v) {
+        int access = 0, tables = 0;
+        const bool ok =
+            cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) ==
+                cudaSuccess;
+        if (!ok) cudaGetLastError();
+        v = ok && access && tables ? 2 : 1;
+        cache[dev].store(v, std::memory_order_relaxed);
+    }
+    return v == 2;
+}
+
+// Largest scenes of the direct slot order.  Copies against direct access, us per
+// call, page-locked buffers: 8,192 particles 102 and 69, 32,768 121 and 94,
+// 110,592 174 and 164, 262,144 279 and 297 (the copies overlap the step).
+// Ordinary memory: 8,192 132 and 78, 32,768 175 and 101, but 110,592 727 and 2133:
+// arrays of that size are unmapped when they are freed, which is slow for pages
+// that the GPU has translated.
+constexpr size_t kDirectPinned = 131072;
+constexpr size_t kDirectPaged = 40000;
+
+// the address under which kernels reach a host buffer, or null; paged is set
+// when it is ordinary (not page-locked) memory
+template <class T>
+T* device_view(T* h, bool& paged) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, h) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (a.type == cudaMemoryTypeHost) return static_cast<T*>(a.devicePointer);
+    if (a.type == cudaMemoryTypeUnregistered && pageable_access()) {
+        paged = true;
+        return h;
+    }
+    return nullptr;       // device or managed memory is no host buffer
+}
+
+// makes the pages of an output buffer present and writable
+void touch_pages(void* p, size_t bytes) {
+    const size_t page = 4096;      // the smallest the system may use
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t k = 0; k < bytes; k += page) c[k] = c[k];
+    if (bytes) c[bytes - 1] = c[bytes - 1];
+}
+}  // namespace
+}  // extern "C++"
+
 static int host_entry(SphgbCtx* ctx, const double* h_pos, const double* h_vel,
                       double* h_pos_out, double* h_vel_out, double* h_rho_out) {
     if (!ctx) return fail(SPHGB_ERR_INVALID, "ctx is null");
@@ -1699,6 +1782,52 @@ static int host_entry(SphgbCtx* ctx, const double* h_pos, const double* h_vel,
     double* sr = ctx->stage + 6 * N;
     const size_t b3 = sizeof(double) * 3 * N;
     const int nb = blocks(ctx->n);
+    const int order = host_order_for_call(ctx);
+    const auto t0 = std::chrono::steady_clock::now();
+    auto record_time = [&]() {
+        const double ms = std::chrono::duration<double, std::milli>(
+                              std::chrono::steady_clock::now() - t0).count();
+        // calls 4 to 6 time the three orders (calls 1 to 3 warm them up)
+        if (ctx->host_order == SPHGB_HOST_ORDER_AUTO && ctx->host_calls >= kAutoTimedFirst &&
+            ctx->host_calls < 2 * kAutoTimedFirst)
+            ctx->host_ms[order] = ms;
+        if (ctx->host_calls < 1000) ++ctx->host_calls;
+    };
+    if (order == SPHGB_HOST_ORDER_SLOT) {
+        // Slot order of small scenes on buffers that kernels can reach
+        // (page-locked, or any host memory where the GPU uses the host's page
+        // tables): no staging copies, no second stream.  The load kernel reads
+        // the rows over the link, the store kernel writes them; the output's
+        // pages are touched here while the step runs, since untouched ones
+        // would fault one by one under the kernel.  See kDirectPinned for why
+        // only small ones.
+        bool paged = false;
+        const double *dp = device_view(h_pos, paged), *dv = device_view(h_vel, paged);
+        double *op = device_view(h_pos_out, paged), *ov = device_view(h_vel_out, paged),
+               *orho = device_view(h_rho_out, paged);
+        if (dp && dv && op && ov && orho && N <= (paged ? kDirectPaged : kDirectPinned)) {
+            k_load_aos<true><<<nb, kBlock, 0, st>>>(ctx->d_scenes, ctx->d_pbegin, ctx->n_scenes, 0, ctx->n,
+                                              dp, dv, ctx->posA, ctx->velA, ctx->pidA, ctx->pos64A);
+            SPHGB_CUDA(cudaGetLastError());
+            int rc = enqueue_step(ctx, st);
+            if (rc) return rc;
+            const bool sep = ctx->out_pos != nullptr;
+            k_slot_of<<<nb, kBlock, 0, st>>>(ctx->d_pbegin, ctx->n_scenes, ctx->n, ctx->pidB,
+                                             ctx->slot_of);
+            SPHGB_CUDA(cudaGetLastError());
+            touch_pages(h_pos_out, b3);
+            touch_pages(h_vel_out, b3);
+            touch_pages(h_rho_out, sizeof(double) * N);
+            k_store_aos<<<nb, kBlock, 0, st>>>(ctx->d_scenes, ctx->d_pbegin, ctx->n_scenes, ctx->n,
+                                               sep ? ctx->out_pos : ctx->posA,
+                                               sep ? ctx->out_vel : ctx->velA, ctx->rho, ctx->slot_of,
+                                               sep ? ctx->out_pos64 : ctx->pos64A, op, ov, orho);
+            SPHGB_CUDA(cudaGetLastError());
+            SPHGB_CUDA(cudaStreamSynchronize(st));
+            record_time();
+            return SPHGB_OK;
+        }
+    }
     // Two streams.  st2 uploads: the positions in kHostPosChunks parts, then
     // the velocities.  st runs the step: each part of the positions is
     // converted and hashed as soon as it is in (the voxel histogram fills in
@@ -1733,7 +1862,7 @@ static int host_entry(SphgbCtx* ctx, const double* h_pos, const double* h_vel,
                                        st2));
             SPHGB_CUDA(cudaEventRecord(e_part, st2));
             SPHGB_CUDA(cudaStreamWaitEvent(st, e_part, 0));
-            k_load_aos<<<blocks(i1 - i0), kBlock, 0, st>>>(ctx->d_scenes, ctx->d_pbegin,
+            k_load_aos<false><<<blocks(i1 - i0), kBlock, 0, st>>>(ctx->d_scenes, ctx->d_pbegin,
                                                             ctx->n_scenes, i0, i1, sp, nullptr,
                                                             ctx->posA, ctx->velA, ctx->pidA,
                                                             ctx->pos64A);
@@ -1741,25 +1870,14 @@ static int host_entry(SphgbCtx* ctx, const double* h_pos, const double* h_vel,
             SPHGB_CUDA(launch_hash_count(L, ctx->posA, ctx->cell, ctx->slot, ctx->vcount, i0, i1));
         }
     }
-    const int order = host_order_for_call(ctx);
     SPHGB_CUDA(cudaMemcpyAsync(sv, h_vel, b3, cudaMemcpyHostToDevice, st2));
     // the pipelined order gathers from the FP64 rows bucket by bucket
     if (order != SPHGB_HOST_ORDER_PIPELINED) {
-        k_load_aos<<<nb, kBlock, 0, st2>>>(ctx->d_scenes, ctx->d_pbegin, ctx->n_scenes, 0, ctx->n,
+        k_load_aos<false><<<nb, kBlock, 0, st2>>>(ctx->d_scenes, ctx->d_pbegin, ctx->n_scenes, 0, ctx->n,
                                            nullptr, sv, ctx->posA, ctx->velA, ctx->pidA, nullptr);
         SPHGB_CUDA(cudaGetLastError());
     }
     SPHGB_CUDA(cudaEventRecord(e_vel, st2));
-    const auto t0 = std::chrono::steady_clock::now();
-    auto record_time = [&]() {
-        const double ms = std::chrono::duration<double, std::milli>(
-                              std::chrono::steady_clock::now() - t0).count();
-        // calls 4 to 6 time the three orders (calls 1 to 3 warm them up)
-        if (ctx->host_order == SPHGB_HOST_ORDER_AUTO && ctx->host_calls >= kAutoTimedFirst &&
-            ctx->host_calls < 2 * kAutoTimedFirst)
-            ctx->host_ms[order] = ms;
-        if (ctx->host_calls < 1000) ++ctx->host_calls;
-    };
     if (order == SPHGB_HOST_ORDER_PIPELINED) {
         int rc = ensure_pipelined(ctx);
         if (!rc) rc = host_step_pipelined(ctx, e_vel, sp, sv, sr, h_pos_out, h_vel_out, h_rho_out);
