@@ -179,6 +179,19 @@ struct SphgbCtx {
     void* owned = nullptr;
     // staging for the host-buffer entry point
     double* stage = nullptr;
+    // neighbour lists of the stage entry points (stage_lists), allocated on their
+    // first call and given back with the scenes they were sized for; apart from
+    // the step's own, which sphgb_ctx_step_neighbours reads after stage calls.
+    // lists_ev: the stream of the last call is done with them.
+    struct {
+        int2* tasks = nullptr;
+        int32_t* words = nullptr;       // 64 counters (tasks, taken, bad), rows, counts
+        int32_t* over = nullptr;
+        bool failed = false;            // no memory: the stages walk
+        cudaEvent_t ev = nullptr;
+        cudaStream_t last = nullptr;
+        bool used = false;
+    } lists;
     // conservation
     int n_chunks = 0;
     ConsChunk* d_chunks = nullptr;
@@ -290,8 +303,17 @@ int dalloc(T** p, size_t count) {
     return SPHGB_OK;
 }
 
+void free_lists(SphgbCtx* c) {
+    if (c->lists.tasks) cudaFree(c->lists.tasks);
+    if (c->lists.words) cudaFree(c->lists.words);
+    if (c->lists.over) cudaFree(c->lists.over);
+    if (c->lists.ev) cudaEventDestroy(c->lists.ev);
+    c->lists = {};
+}
+
 void free_ctx(SphgbCtx* c) {
     if (!c) return;
+    free_lists(c);
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
     void* ptrs[] = {c->d_scenes, c->d_scenes_ref, c->d_pbegin, c->d_pipe, c->cell, c->slot_of, c->slot, c->tmp_pid,
                     c->vstart, c->counts, c->posB, c->velB, c->pidB,
@@ -820,6 +842,73 @@ int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int rang
     return SPHGB_OK;
 }
 
+// Neighbour lists of the sorted state and voxel table of a stage call, by the
+// step's density passes, which also write the densities when rho is given.
+// Returns the lists, or empty ones where the stage has to walk as it did before
+// there were lists: under stream capture (the first call allocates, and calls
+// are ordered by an event) and without memory.  Lists of a table that is not
+// the state's are vetoed on the device.
+int stage_lists(SphgbCtx* c, const Launch& L, const float4* pos, const int32_t* vstart,
+                const int32_t* vcount, float* rho, NbrList& out, int32_t*& bad) {
+    out = NbrList{};
+    bad = nullptr;
+    const size_t N = (size_t)c->n;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(L.stream, &cap) != cudaSuccess) {
+        cudaGetLastError();       // the legacy stream beside a capture elsewhere
+        return SPHGB_OK;
+    }
+    auto& l = c->lists;
+    if (cap != cudaStreamCaptureStatusNone || l.failed || N == 0) return SPHGB_OK;
+    const size_t head = kCountersPad;
+    if (!l.words) {
+        // allowed beside a capture of another stream or thread
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        int rc = dalloc(&l.tasks, N);
+        if (!rc) rc = dalloc(&l.words, head + (kListCap + 1) * N + 8);
+        if (!rc && c->uncapped) rc = dalloc(&l.over, 8 * (size_t)std::min(N * kOverPerParticle, kOverMax));
+        if (!rc && cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            rc = SPHGB_ERR_CUDA;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc) {
+            free_lists(c);
+            l.failed = true;
+            g_last_error.clear();
+            return SPHGB_OK;
+        }
+    }
+    if (l.used && l.last != L.stream) SPHGB_CUDA(cudaStreamWaitEvent(L.stream, l.ev, 0));
+    l.used = true;
+    l.last = L.stream;
+    SPHGB_CUDA(cudaMemsetAsync(l.words, 0, sizeof(int32_t) * head, L.stream));
+    bad = l.words + 2;
+    out.idx = l.words + head;
+    out.count = out.idx + kListCap * N;
+    out.veto = bad;
+    if (c->uncapped) {
+        out.over = l.over;
+        out.over_used = reinterpret_cast<unsigned long long*>(l.words + kOverCounter);
+        out.over_units = std::min(N * kOverPerParticle, kOverMax);
+    }
+    SPHGB_CUDA(launch_stage_tasks(L, pos, vstart, vcount, l.tasks, l.words, bad));
+    // dense scenes: see density_pass
+    if (c->density_pass() == SphgbCtx::kPassWc)
+        SPHGB_CUDA(launch_density_wc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks,
+                                     l.words, l.words + 1));
+    else
+        SPHGB_CUDA(launch_density_tc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks, 1,
+                                     l.words, l.words + 1, c->uncapped));
+    return SPHGB_OK;
+}
+// the stage is done with the lists
+int stage_lists_end(SphgbCtx* c, const NbrList& l, cudaStream_t st) {
+    if (l.count) SPHGB_CUDA(cudaEventRecord(c->lists.ev, st));
+    return SPHGB_OK;
+}
+
 // checked mode: validate the step just enqueued (inputs in the B buffers,
 // outputs where enqueue_forces wrote them)
 int enqueue_checks(SphgbCtx* c, cudaStream_t st) {
@@ -1037,6 +1126,7 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
         cudaFree(c->stage);
         c->stage = nullptr;
     }
+    free_lists(c);
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
     c->graphs.clear();
     return SPHGB_OK;
@@ -2136,10 +2226,16 @@ int sphgb_density(SphgbCtx* ctx, const float* d_pos_sorted, const int32_t* d_vox
     if (!ctx) return fail(SPHGB_ERR_INVALID, "ctx is null");
     if (ctx->n > 0 && (!d_pos_sorted || !d_rho_out)) return fail(SPHGB_ERR_INVALID, "null buffer");
     cudaStream_t st = as_stream(stream);
-    SPHGB_CUDA(launch_density(ctx->launch(st, true), reinterpret_cast<const float4*>(d_pos_sorted),
-                              nullptr, d_voxel_start, d_voxel_count, d_rho_out, nullptr,
-                              NbrList{}));
-    return SPHGB_OK;
+    const Launch L = ctx->launch(st, true);
+    const float4* pos = reinterpret_cast<const float4*>(d_pos_sorted);
+    NbrList nbr;
+    int32_t* bad;
+    int rc = stage_lists(ctx, L, pos, d_voxel_start, d_voxel_count, d_rho_out, nbr, bad);
+    if (rc) return rc;
+    // without lists, or when they were vetoed: one thread walks per particle
+    SPHGB_CUDA(launch_density(L, pos, nullptr, d_voxel_start, d_voxel_count, d_rho_out, nullptr,
+                              NbrList{}, bad));
+    return stage_lists_end(ctx, nbr, st);
 }
 
 int sphgb_forces(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel_sorted,
@@ -2155,11 +2251,16 @@ int sphgb_forces(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel_so
     SPHGB_CUDA(launch_force_inputs(L, reinterpret_cast<const float4*>(d_pos_sorted),
                                    reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted,
                                    ctx->fin));
+    NbrList nbr;
+    int32_t* bad;
+    int rc = stage_lists(ctx, L, reinterpret_cast<const float4*>(d_pos_sorted), d_voxel_start,
+                         d_voxel_count, nullptr, nbr, bad);
+    if (rc) return rc;
     SPHGB_CUDA(launch_forces(L, reinterpret_cast<const float4*>(d_pos_sorted),
                              reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted, ctx->fin,
                              d_voxel_start, d_voxel_count, reinterpret_cast<float4*>(d_pressure_out),
-                             reinterpret_cast<float4*>(d_viscosity_out)));
-    return SPHGB_OK;
+                             reinterpret_cast<float4*>(d_viscosity_out), nbr));
+    return stage_lists_end(ctx, nbr, st);
 }
 
 int sphgb_integrate(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel_sorted,
@@ -2179,14 +2280,19 @@ int sphgb_integrate(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel
     SPHGB_CUDA(launch_force_inputs(L, reinterpret_cast<const float4*>(d_pos_sorted),
                                    reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted,
                                    ctx->fin));
+    NbrList nbr;
+    int32_t* bad;
+    int rc = stage_lists(ctx, L, reinterpret_cast<const float4*>(d_pos_sorted), d_voxel_start,
+                         d_voxel_count, nullptr, nbr, bad);
+    if (rc) return rc;
     SPHGB_CUDA(launch_integrate(L, reinterpret_cast<const float4*>(d_pos_sorted),
                                 reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted,
                                 ctx->fin, d_pid_sorted, d_pos64_sorted, d_voxel_start,
-                                d_voxel_count, d_scene_step, NbrList{},
+                                d_voxel_count, d_scene_step, nbr,
                                 reinterpret_cast<float4*>(d_pos_out),
                                 reinterpret_cast<float4*>(d_vel_out), d_pid_out, d_pos64_out,
                                 reinterpret_cast<float4*>(d_force_out)));
-    return SPHGB_OK;
+    return stage_lists_end(ctx, nbr, st);
 }
 
 int sphgb_pipe_find_segment(const double* d_pos, int n, const double* d_pipe, int pipe_rows,

@@ -384,7 +384,8 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const int lane = threadIdx.x & 31;
     TcShared& S = sh[threadIdx.x >> 5];
     const unsigned lt = (1u << lane) - 1u;
-    const int n_tasks = *grid_wait(task_count);
+    int n_tasks = *grid_wait(task_count);
+    if (nbr.veto && *after_wait(nbr.veto)) n_tasks = 0;
     // A warp's first task is its own number; each later one comes from a
     // counter (the cost of a task varies with its voxel's neighbourhood, and a
     // fixed share per warp left warps idle at the end of the pass, 15 % of its
@@ -593,8 +594,8 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             if (!over) acc.merge(rest);
             if (home) {
                 const float r = (acc.s * sc.w_const) * sc.mass;
-                rho[s] = r;
-                write_force_inputs(s, pi, sc, vel, r, fin);
+                if (rho) rho[s] = r;
+                if (fin) write_force_inputs(s, pi, sc, vel, r, fin);
                 if (nbr.count) nbr.count[s] = over ? -1 : others;
             }
         }

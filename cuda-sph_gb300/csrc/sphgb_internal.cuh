@@ -567,11 +567,15 @@ struct NbrList {
     int32_t* over = nullptr;
     unsigned long long* over_used = nullptr;    // units taken, zero before the density pass
     unsigned long long over_units = 0;
+    // set on the device when the lists were not built (launch_stage_tasks):
+    // every particle then counts as having none
+    const int32_t* veto = nullptr;
 };
 // the list of a particle: its row, or its place in the pool; cnt -1: none
 __device__ __forceinline__ const int32_t* nbr_row(const NbrList& nbr, int s, int& cnt) {
     const int32_t* row = nbr.idx ? nbr.idx + (size_t)s * kListCap : nullptr;
-    if (cnt < 0 && nbr.over) {
+    if (nbr.veto && __ldg(nbr.veto)) cnt = -1;
+    else if (cnt < 0 && nbr.over) {
         const int2 e = __ldg(reinterpret_cast<const int2*>(row));
         if (e.x > 0) {
             cnt = e.x;
@@ -707,9 +711,18 @@ cudaError_t launch_rank_gather(const Launch& L, const int32_t* cell, const int32
                                TaskLists tasks = TaskLists{});
 // fin (optional, with vel): the force inputs of each particle, two float4
 // per particle: (x, y, z, p/rho^2) and (vx, vy, vz, 1/rho)
+// only_if (device, optional): the pass runs when the word is not zero
 cudaError_t launch_density(const Launch& L, const float4* pos, const float4* vel,
                            const int32_t* vstart, const int32_t* vcount, float* rho,
-                           float4* fin, NbrList nbr);
+                           float4* fin, NbrList nbr, const int32_t* only_if = nullptr);
+// Density tasks of a sorted state and voxel table that a caller brings (the
+// stage entry points), as the rank-gather lists them.  bad is set, and the
+// density passes given nbr.veto = bad do nothing, when the table is not that
+// of the state: some particle's slot outside its voxel's range, or a range that
+// is not one voxel's.
+cudaError_t launch_stage_tasks(const Launch& L, const float4* pos, const int32_t* vstart,
+                               const int32_t* vcount, int2* tasks, int32_t* task_count,
+                               int32_t* bad);
 // the step's density pass: one warp per task (<= kTaskRun particles of one voxel);
 // task_next: a zeroed counter from which the warps take the tasks
 // task_offset (optional, device): the tasks start at tasks[*task_offset] (one
@@ -735,7 +748,8 @@ cudaError_t launch_gather_vel(const Launch& L, const int32_t* pid, const float4*
                               const float* rho, float4* vel_out, float4* fin);
 cudaError_t launch_forces(const Launch& L, const float4* pos, const float4* vel,
                           const float* rho, const float4* fin, const int32_t* vstart,
-                          const int32_t* vcount, float4* pressure, float4* viscosity);
+                          const int32_t* vcount, float4* pressure, float4* viscosity,
+                          NbrList nbr = NbrList{});
 cudaError_t launch_integrate(const Launch& L, const float4* pos, const float4* vel,
                              const float* rho, const float4* fin, const int32_t* pid,
                              const double* pos64, const int32_t* vstart, const int32_t* vcount,

@@ -81,7 +81,7 @@ __device__ __forceinline__ void density_one(int s, const float4& pi, const Scene
         });
     }
     const float r = (acc.s * sc.w_const) * sc.mass;
-    rho[s] = r;
+    if (rho) rho[s] = r;
     if (fin) write_force_inputs(s, pi, sc, vel, r, fin);
     if (nbr.count) nbr.count[s] = others <= kListCap ? others : -1;
 }
@@ -94,8 +94,10 @@ k_density(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegi
           int n, const float4* __restrict__ pos, const float4* __restrict__ vel,
           const int32_t* __restrict__ vstart, const int32_t* __restrict__ vcount,
           float* __restrict__ rho, float4* __restrict__ fin, NbrList nbr,
-          const int32_t* __restrict__ step_limit, const int32_t* __restrict__ scene_step) {
+          const int32_t* __restrict__ step_limit, const int32_t* __restrict__ scene_step,
+          const int32_t* __restrict__ only_if) {
     __shared__ int32_t s_list[kListCap][kBlock];
+    if (only_if && !*only_if) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int si = scene_of(s, pbegin, n_scenes);
@@ -263,7 +265,8 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const int lane = threadIdx.x & 31;
     WcShared& S = sh[threadIdx.x >> 5];
     const unsigned lt = (1u << lane) - 1u;
-    const int n_tasks = *grid_wait(task_count);
+    int n_tasks = *grid_wait(task_count);
+    if (nbr.veto && *after_wait(nbr.veto)) n_tasks = 0;
     if (task_offset) tasks += *after_wait(task_offset);   // one bucket of a bucketed task list
     // A warp's first task is its own number; each later one comes from a
     // counter (the cost of a task varies with its voxel's neighbourhood, and a
@@ -417,7 +420,7 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             acc.merge(rest);
             if (home) {
                 const float r = (acc.s * sc.w_const) * sc.mass;
-                rho[s] = r;
+                if (rho) rho[s] = r;
                 if (kGather) {
                     const float4 v = vel_row(vrows, s, pbegin, n_scenes);
                     vrows.vel_out[s] = v;
@@ -432,6 +435,33 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         __syncwarp();
         if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
     }
+}
+
+// see launch_stage_tasks; one thread per slot
+__global__ void __launch_bounds__(kBlock)
+k_stage_tasks(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin, int n_scenes,
+              int n, const float4* __restrict__ pos, const int32_t* __restrict__ vstart,
+              const int32_t* __restrict__ vcount, int2* __restrict__ tasks,
+              int32_t* __restrict__ task_count, int32_t* __restrict__ bad) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const SceneDev& sc = scenes[scene_of(s, pbegin, n_scenes)];
+    auto voxel = [&](int slot) {
+        const float4 p = __ldg(pos + slot);
+        if (!finite3(p)) return sc.v_begin + sc.v_count;
+        return sc.v_begin + voxel_index(voxel_coord(p.x, sc.vs[0], sc.dims[0]),
+                                        voxel_coord(p.y, sc.vs[1], sc.dims[1]),
+                                        voxel_coord(p.z, sc.vs[2], sc.dims[2]), sc.tiled, sc.dims[0],
+                                        sc.dims[1], sc.nt0, sc.nt1);
+    };
+    const int vid = voxel(s);
+    const int st = __ldg(vstart + vid), c = __ldg(vcount + vid);
+    // the slot in its voxel's range, the range inside the scene; the slot before
+    // it in the same voxel; and the range's last slot, seen from its first
+    bool ok = s >= st && s - st < c && st >= sc.p_begin && c <= sc.p_begin + sc.p_count - st;
+    if (ok) ok = s > st ? voxel(s - 1) == vid : voxel(st + c - 1) == vid;
+    if (!ok) atomicOr(bad, 1);
+    else if ((s - st) % kTaskRun == 0) tasks[atomicAdd(task_count, 1)] = make_int2(vid, s);
 }
 
 // Velocities of a state loaded in original particle order (scene offset + id)
@@ -666,7 +696,7 @@ k_forces(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin
          int n, const float4* __restrict__ pos, const float4* __restrict__ vel,
          const float4* __restrict__ fin, const int32_t* __restrict__ vstart,
          const int32_t* __restrict__ vcount, float4* __restrict__ pressure,
-         float4* __restrict__ viscosity) {
+         float4* __restrict__ viscosity, NbrList nbr) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const SceneDev& sc = scenes[scene_of(s, pbegin, n_scenes)];
@@ -675,7 +705,9 @@ k_forces(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin
     float4 fa, fb;
     ldg256(fin + 2 * s, fa, fb);
     const float2 ai = make_float2(fa.w, fb.w);
-    const Forces f = forces_of(s, pi, vi, ai, sc, pos, fin, vstart, vcount, nullptr, n, -1);
+    int cnt = nbr.count ? __ldg(nbr.count + s) : -1;
+    const int32_t* list = nbr_row(nbr, s, cnt);
+    const Forces f = forces_of(s, pi, vi, ai, sc, pos, fin, vstart, vcount, list, n, cnt);
     const float vscale = sc.mass * sc.visc * ai.y;
     pressure[s] = make_float4(f.p[0], f.p[1], f.p[2], 0.0f);
     viscosity[s] = make_float4(visc_term(f, 0, vscale), visc_term(f, 1, vscale),
@@ -1021,12 +1053,12 @@ k_neighbours(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
 
 cudaError_t launch_density(const Launch& L, const float4* pos, const float4* vel,
                            const int32_t* vstart, const int32_t* vcount, float* rho,
-                           float4* fin, NbrList nbr) {
+                           float4* fin, NbrList nbr, const int32_t* only_if) {
     if (L.n == 0) return cudaSuccess;
     auto kernel = L.layout == 1 ? k_density<1> : L.layout == 2 ? k_density<2> : k_density<0>;
     kernel<<<blocks_for(L.n), kBlock, 0, L.stream>>>(L.scenes, L.pbegin, L.n_scenes, L.n, pos, vel,
                                                      vstart, vcount, rho, fin, nbr, L.step_limit,
-                                                     L.scene_step);
+                                                     L.scene_step, only_if);
     return cudaGetLastError();
 }
 
@@ -1054,6 +1086,15 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
     return launch_chained(kernel, blocks, kWcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
                           L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, task_count, task_next,
                           task_offset, vrows);
+}
+
+cudaError_t launch_stage_tasks(const Launch& L, const float4* pos, const int32_t* vstart,
+                               const int32_t* vcount, int2* tasks, int32_t* task_count,
+                               int32_t* bad) {
+    if (L.n == 0) return cudaSuccess;
+    k_stage_tasks<<<blocks_for(L.n), kBlock, 0, L.stream>>>(L.scenes, L.pbegin, L.n_scenes, L.n, pos,
+                                                            vstart, vcount, tasks, task_count, bad);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_gather_vel(const Launch& L, const int32_t* pid, const float4* vel_in,
@@ -1086,12 +1127,13 @@ cudaError_t launch_force_inputs(const Launch& L, const float4* pos, const float4
 
 cudaError_t launch_forces(const Launch& L, const float4* pos, const float4* vel,
                           const float* rho, const float4* fin, const int32_t* vstart,
-                          const int32_t* vcount, float4* pressure, float4* viscosity) {
+                          const int32_t* vcount, float4* pressure, float4* viscosity,
+                          NbrList nbr) {
     (void)rho;
     if (L.n == 0) return cudaSuccess;
     k_forces<<<blocks_for(L.n), kBlock, 0, L.stream>>>(L.scenes, L.pbegin, L.n_scenes, L.n, pos,
                                                         vel, fin, vstart, vcount, pressure,
-                                                        viscosity);
+                                                        viscosity, nbr);
     return cudaGetLastError();
 }
 
