@@ -221,22 +221,18 @@ k_scatter(int n, const int32_t* __restrict__ cell, const int32_t* __restrict__ s
 // member ids ascending with a bitonic network whose comparators all put the
 // smaller value at the lower index, so the segment is padded to a power of
 // two implicitly (comparators reaching past the end are no-ops).  Segments up
-// to kSmemSort ids are sorted in shared memory, longer ones in place in global
-// memory.
+// to kSmemSort ids are sorted in shared memory, longer ones in tiles of that
+// size with the long comparators in global memory.
 constexpr int kSortThreads = 1024;
 constexpr int kSmemSort = 8192;
 
 __device__ __forceinline__ void bitonic_pass(int32_t* a, int c, int n2, int k, int j) {
     const int half = n2 >> 1;
     for (int t = threadIdx.x; t < half; t += kSortThreads) {
-        int i, p;
-        if (j == (k >> 1)) {            // first step of a merge: mirror within the k-block
-            i = (t / j) * k + (t % j);
-            p = i ^ (k - 1);
-        } else {                        // half-cleaner
-            i = (t / j) * 2 * j + (t % j);
-            p = i + j;
-        }
+        // j is a power of two: i = (t / j) 2 j + t % j.  The first step of a
+        // merge mirrors within the k-block, the others are half-cleaners.
+        const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
+        const int p = j == (k >> 1) ? i ^ (k - 1) : i + j;
         if (p < c) {
             const int32_t x = a[i], y = a[p];
             if (y < x) { a[i] = y; a[p] = x; }
@@ -248,8 +244,10 @@ __device__ __forceinline__ void bitonic_pass(int32_t* a, int c, int n2, int k, i
 // network: every id counts the smaller ones (the ids are distinct), from shared
 // memory four at a time, all threads reading the same quad.  A network of 1024
 // threads per voxel spends its time in barriers (36 for 133 ids): the 4,000
-// voxels of ~133 particles of the 262,144-particle pipe took 86 us, 7 us this way.
-constexpr int kRankSort = 1024;
+// voxels of ~133 particles of the 262,144-particle pipe took 86 us, 13 us this
+// way.  Beyond 512 ids the counting grows past the network (the pipe's later
+// steps, voxels of 600 to 3,000: the sort 74 us with a limit of 1024, 49 with 512).
+constexpr int kRankSort = 512;
 constexpr int kQuarter = kSortThreads / 4;
 
 __device__ __forceinline__ void quarter_sync(int quarter) {
@@ -264,14 +262,10 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
     const int nb = *grid_wait(big_count);
     const int quarter = threadIdx.x / kQuarter, t = threadIdx.x % kQuarter;
     int32_t* sq = sm + quarter * kRankSort;
-    bool any_long = false;
     for (int b = blockIdx.x * 4 + quarter; b < nb; b += gridDim.x * 4) {
         const int vid = big_list[b];
         const int st = vstart[vid], c = vcount[vid];
-        if (c > kRankSort) {
-            any_long = true;
-            continue;
-        }
+        if (c > kRankSort) continue;
         const int c4 = (c + 3) & ~3;
         for (int i = t; i < c4; i += kQuarter) sq[i] = i < c ? tmp_pid[st + i] : INT_MAX;
         quarter_sync(quarter);
@@ -286,28 +280,44 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
         }
         quarter_sync(quarter);
     }
-    // the longer ones of these voxels, one after another by the whole block
+    // the longer ones, a whole block each (other voxels than the quarters': four
+    // long ones of one block would wait for one another)
+    bool any_long = false;
+    for (int b = blockIdx.x + threadIdx.x * gridDim.x; b < nb; b += kSortThreads * gridDim.x)
+        any_long |= vcount[big_list[b]] > kRankSort;
     if (!__syncthreads_or(any_long)) return;
-    for (int b0 = blockIdx.x * 4; b0 < nb; b0 += gridDim.x * 4) {
-        for (int b = b0; b < min(nb, b0 + 4); ++b) {
-            const int vid = big_list[b];
-            const int st = vstart[vid], c = vcount[vid];
-            if (c <= kRankSort) continue;
-            int n2 = 1;
-            while (n2 < c) n2 <<= 1;
-            const bool in_smem = n2 <= kSmemSort;
-            int32_t* a = in_smem ? sm : tmp_pid + st;
-            if (in_smem)
-                for (int i = threadIdx.x; i < c; i += kSortThreads) sm[i] = tmp_pid[st + i];
-            __syncthreads();
-            for (int k = 2; k <= n2; k <<= 1)
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    bitonic_pass(a, c, n2, k, j);
-                    __syncthreads();
-                }
-            if (in_smem)
-                for (int i = threadIdx.x; i < c; i += kSortThreads) tmp_pid[st + i] = sm[i];
-            __syncthreads();
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        const int vid = big_list[b];
+        const int st = vstart[vid], c = vcount[vid];
+        if (c <= kRankSort) continue;
+        int n2 = 1;
+        while (n2 < c) n2 <<= 1;
+        // A network's blocks of up to kSmemSort ids stay inside one aligned
+        // tile, so a tile runs all its steps in shared memory, and only the
+        // comparators that reach further work in global memory: 15 of the 171
+        // passes over 262,144 ids.
+        int32_t* a = tmp_pid + st;
+        auto in_tiles = [&](int k0, int k1, int j_top) {
+            for (int base = 0; base < c; base += kSmemSort) {
+                const int m = min(kSmemSort, c - base);
+                for (int i = threadIdx.x; i < m; i += kSortThreads) sm[i] = a[base + i];
+                __syncthreads();
+                for (int k = k0; k <= k1; k <<= 1)
+                    for (int j = min(k >> 1, j_top); j > 0; j >>= 1) {
+                        bitonic_pass(sm, m, min(n2, kSmemSort), k, j);
+                        __syncthreads();
+                    }
+                for (int i = threadIdx.x; i < m; i += kSortThreads) a[base + i] = sm[i];
+                __syncthreads();
+            }
+        };
+        in_tiles(2, min(n2, kSmemSort), kSmemSort);
+        for (int k = 2 * kSmemSort; k <= n2; k <<= 1) {
+            for (int j = k >> 1; j >= kSmemSort; j >>= 1) {
+                bitonic_pass(a, c, n2, k, j);
+                __syncthreads();
+            }
+            in_tiles(k, k, kSmemSort / 2);
         }
     }
 }

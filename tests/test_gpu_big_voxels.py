@@ -1,5 +1,5 @@
 """Voxels above the big-voxel threshold: their ids are sorted by counting up to
-1024 members and by a sorting network beyond; the organised state is the
+512 members and by a sorting network beyond; the organised state is the
 reference's (voxel, particle id) order whatever the input order."""
 import numpy as np
 import pytest
@@ -9,8 +9,9 @@ from gpu_util import to_device, torch_cuda
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("sizes", [(64, 65, 66), (255, 256, 257, 1, 0, 3), (1023, 1024, 1025),
-                                   (2048, 5, 2049, 70), (9000, 100, 8192, 1024, 77),
+@pytest.mark.parametrize("sizes", [(64, 65, 66), (255, 256, 257, 1, 0, 3), (511, 512, 513, 1023, 1024, 1025),
+                                   (2048, 5, 2049, 70), (9000, 100, 8192, 1024, 77), (8193,), (16384, 16385), (40_000, 3, 1200),
+                                   (100_000,),
                                    tuple([133] * 40 + [1500] + [200] * 30)])
 def test_order_of_big_voxels(sizes):
     torch = torch_cuda()
