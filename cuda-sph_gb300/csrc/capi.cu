@@ -85,7 +85,7 @@ constexpr double kTileMaxOccupancy = 8.0;   // particles per voxel, table mean
 constexpr int kHostRanges = 8;
 // the pipelined host order: ranges of the force pass and buckets of the
 // density pass (host_step_pipelined)
-constexpr int kPipeRanges = 16;
+constexpr int kPipeRanges = 7;
 constexpr int kHostFirstRangeEvent = 6;
 // the host entry uploads the positions in kHostPosChunks parts; each is
 // converted and hashed while the next one is in flight
@@ -223,15 +223,15 @@ struct SphgbCtx {
     // density tasks bucketed by the original-index range of their first
     // particle and the slots of each bucket's tasks, the latest bucket each
     // voxel's tasks fall in, the counters, offsets and dependencies (on the
-    // device and page-locked), two more streams and their events
+    // device and page-locked), one more stream and the events
     int2* tasks_b = nullptr;
     int32_t* slots_b = nullptr;
     int32_t* vbucket = nullptr;
     int32_t* pipe_i = nullptr;
     int32_t* h_pipe = nullptr;
     size_t cap_tasks_b = 0, cap_vbucket = 0;
-    cudaStream_t host_stream3 = nullptr, host_stream4 = nullptr;
-    cudaEvent_t pipe_ev[3 + 2 * kPipeRanges] = {};
+    cudaStream_t host_stream4 = nullptr;
+    cudaEvent_t pipe_ev[3 + kPipeRanges] = {};
     std::map<int, cudaGraphExec_t> graphs;
 
     // Which density pass takes the step's tasks: k_density_tc those of sparse
@@ -325,7 +325,6 @@ void free_ctx(SphgbCtx* c) {
     if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
     if (c->host_stream) cudaStreamDestroy(c->host_stream);
     if (c->host_stream2) cudaStreamDestroy(c->host_stream2);
-    if (c->host_stream3) cudaStreamDestroy(c->host_stream3);
     if (c->host_stream4) cudaStreamDestroy(c->host_stream4);
     for (cudaEvent_t e : c->pipe_ev)
         if (e) cudaEventDestroy(e);
@@ -1364,26 +1363,32 @@ namespace {
 // of range r.  Force bucket b needs the densities and force
 // records of every neighbour of its particles, all of which lie in the 27
 // walk voxels around their voxels: dep[b] is the latest bucket of any task in
-// those voxels, and force bucket b starts as soon as density buckets
-// 0..dep[b] and their velocity gathers are done, while later buckets are
-// still in the density pass.  When particle ids follow space (a lattice in
-// index order), dep[b] is about b + 1 and the downloads overlap most of the
-// density pass; when they do not, dep[b] is the last bucket and the downloads
-// wait for the whole density pass.
+// those voxels, and force bucket b comes right after density bucket dep[b].
+// When particle ids follow space (a lattice in index order), dep[b] is about
+// b + 1 and the downloads overlap most of the density pass; when they do not,
+// dep[b] is the last bucket and the downloads wait for the whole density pass.
+//
+// One stream computes.  With the force buckets on a stream of their own beside
+// 16 density buckets, the kernels of both passes shared the SMs, and the force
+// pass the small L1 that a density block leaves it; in a row, with fewer and
+// larger launches, each kernel has the chip.  4,194,304 particles, ms per call:
+// 2.99 on two streams (k_density_wc; 3.06 with k_density_tc), in a row 2.87; with
+// 6 buckets 2.88, 8 2.89, 10 2.94, 4 3.06.
 // pipe_i layout (kPipeK entries each): task counts per bucket, task fill
 // counters, task counters of the density launches, dep, task offsets, slot
 // counts, slot fill counters, slot offsets, dl.
 constexpr int kPipeK = kPipeRanges;
 constexpr int kPipeInts = 9 * kPipeK;
-// The first buckets run while the velocities are still on the host link and
-// are gathered by their own kernel; later buckets wait for the upload (done
-// by then at 4M) and gather their velocities in the density pass itself.
-constexpr int kPipeGathered = 2;
+// The first bucket runs while the velocities are still on the host link and is
+// gathered by a kernel of its own; later buckets wait for the upload (done by
+// then at 4M) and gather their velocities in the density pass itself (2.97 ->
+// 2.91 ms per call).
+constexpr int kPipeGathered = 1;
 
 // Range r of the original indices is [b[r], b[r + 1]).  The last ranges are
 // smaller: the force buckets and downloads that must wait for the end of the
 // density pass are short.  Relative sizes of the ranges:
-constexpr int kPipeWeight[kPipeK] = {4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 2, 1, 1};
+constexpr int kPipeWeight[kPipeK] = {4, 4, 4, 4, 4, 2, 1};
 struct PipeBounds {
     int32_t b[kPipeK + 1];
 };
@@ -1549,7 +1554,7 @@ __global__ void k_bucket_deps(const SceneDev* __restrict__ scenes, const int2* _
 // and the force pass runs only the tasks' slots).
 bool pipelined_eligible(const SphgbCtx* c) {
     return c->n_scenes == 1 && !c->h_scenes[0].walk_trunc && c->h_scenes[0].cap <= kListCap &&
-           c->density_variant == SPHGB_DENSITY_WARP && c->n >= 32 * kPipeK && !c->step_limit;
+           c->density_variant == SPHGB_DENSITY_WARP && c->n >= 512 && !c->step_limit;
 }
 
 int ensure_pipelined(SphgbCtx* c) {
@@ -1579,13 +1584,6 @@ int ensure_pipelined(SphgbCtx* c) {
     }
     if (!c->h_pipe) SPHGB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&c->h_pipe),
                                              sizeof(int32_t) * kPipeInts, cudaHostAllocDefault));
-    if (!c->host_stream3) {
-        // the gathers and force buckets go ahead of the density buckets when
-        // both have blocks waiting for an SM
-        int least = 0, greatest = 0;
-        SPHGB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        SPHGB_CUDA(cudaStreamCreateWithPriority(&c->host_stream3, cudaStreamNonBlocking, greatest));
-    }
     if (!c->host_stream4)
         SPHGB_CUDA(cudaStreamCreateWithFlags(&c->host_stream4, cudaStreamNonBlocking));
     for (cudaEvent_t& e : c->pipe_ev)
@@ -1596,40 +1594,28 @@ int ensure_pipelined(SphgbCtx* c) {
 // The host entry after the positions have been hashed (st) and the
 // velocities uploaded (st2, event e_vel): the step with its force pass and
 // downloads pipelined behind the density pass (see kPipeK above).  st sorts,
-// buckets the tasks and runs the density buckets; st3, which has the
-// greatest priority, builds the slot map, gathers the first buckets'
-// velocities and runs the force buckets, each after the density buckets it
-// depends on; st4 reads the counts and dependencies back and downloads each
-// range's rows.
+// buckets the tasks and runs the density and force buckets; st4 finds the
+// dependencies, reads them and the counts back and downloads each range's rows.
 int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, double* sr,
                         double* h_pos_out, double* h_vel_out, double* h_rho_out) {
     const size_t N = (size_t)c->n;
-    cudaStream_t st = c->host_stream, st3 = c->host_stream3, st4 = c->host_stream4;
-    cudaEvent_t e_org = c->pipe_ev[0], e_bk = c->pipe_ev[1], e_dep = c->pipe_ev[2];
-    cudaEvent_t* e_bucket = c->pipe_ev + 3;
-    cudaEvent_t* e_range = c->pipe_ev + 3 + kPipeK;
-    Launch L = c->launch(st), L3 = c->launch(st3);
-    // blocks that wait for the density bucket before theirs would hold the SM
-    // slots that the force buckets take meanwhile
-    L.chained = L3.chained = false;
+    cudaStream_t st = c->host_stream, st4 = c->host_stream4;
+    cudaEvent_t e_bk = c->pipe_ev[1], e_dep = c->pipe_ev[2];
+    cudaEvent_t* e_range = c->pipe_ev + 3;
+    const Launch L = c->launch(st);
     double* p64A = c->any_pipe ? c->pos64A : nullptr;
     double* p64B = c->any_pipe ? c->pos64B : nullptr;
-    // sort (the velocities follow bucket by bucket: gathered into slot order
-    // by the density buckets themselves, or for the first buckets by a kernel
-    // of their own on st3)
+    // sort (the velocities follow bucket by bucket: gathered into slot order by
+    // the density buckets themselves, or for the first one by its own kernel)
     TaskLists whole;
     whole.list = c->tasks;
     whole.count = c->big_count + 1;
     int rc = enqueue_organize(c, L, c->posA, nullptr, c->pidA, p64A, c->posB, c->velB, c->pidB,
                               p64B, c->vstart, c->vcount, nullptr, whole, true);
     if (rc) return rc;
-    SPHGB_CUDA(cudaEventRecord(e_org, st));
-    // st3 after the sort and the velocity upload: the gathers and the
-    // density buckets read the upload's FP64 rows, and a force bucket
-    // overwrites only the rows of its own particles, whose velocities its
-    // density bucket (or gather) has already read
-    SPHGB_CUDA(cudaStreamWaitEvent(st3, e_org, 0));
-    SPHGB_CUDA(cudaStreamWaitEvent(st3, e_vel, 0));
+    // The gathers and the density buckets read the upload's FP64 rows; a force
+    // bucket overwrites only the rows of its own particles, whose velocities its
+    // density bucket (or gather) has already read.
     // buckets and dependencies
     int32_t* pi = c->pipe_i;
     const int32_t* n_tasks = c->big_count + 1;
@@ -1653,23 +1639,36 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
     SPHGB_CUDA(cudaMemcpyAsync(c->h_pipe, pi, sizeof(int32_t) * kPipeInts,
                                cudaMemcpyDeviceToHost, st4));
     SPHGB_CUDA(cudaEventRecord(e_dep, st4));
-    // The density buckets, one after another on st.  From bucket
-    // kPipeGathered on they wait for the velocity upload and gather their
-    // velocities themselves.
+    // One compute stream: density bucket b with its velocities, then every force
+    // bucket whose neighbours are now all there.
     VelRows vrows;
     vrows.vel64 = sv;
     vrows.pid = c->pidB;
     vrows.vel_out = c->velB;
-    for (int b = 0; b < kPipeK; ++b) {
-        if (b == kPipeGathered) SPHGB_CUDA(cudaStreamWaitEvent(st, e_vel, 0));
-        // k_density_wc, also for sparse scenes: in short launches beside the
-        // force buckets k_density_tc measured 3.06 ms per call against 2.98
-        SPHGB_CUDA(launch_density_wc(L, c->posB, nullptr, c->vstart, c->vcount, c->rho, c->fin,
-                                     c->nbr, c->tasks_b, pi + b, pi + 2 * kPipeK + b,
-                                     pi + 4 * kPipeK + b,
-                                     b >= kPipeGathered ? vrows : VelRows{}));
-        SPHGB_CUDA(cudaEventRecord(e_bucket[b], st));
-    }
+    int b_density = 0;
+    auto density_through = [&](int last) -> int {
+        for (; b_density <= last; ++b_density) {
+            const int b = b_density;
+            const VelRows vr = b < kPipeGathered ? VelRows{} : vrows;
+            if (b == kPipeGathered) SPHGB_CUDA(cudaStreamWaitEvent(st, e_vel, 0));
+            if (c->density_pass() == SphgbCtx::kPassTc)
+                SPHGB_CUDA(launch_density_tc(L, c->posB, nullptr, c->vstart, c->vcount, c->rho,
+                                             c->fin, c->nbr, c->tasks_b, 1, pi + b,
+                                             pi + 2 * kPipeK + b, false, pi + 4 * kPipeK + b, vr));
+            else
+                SPHGB_CUDA(launch_density_wc(L, c->posB, nullptr, c->vstart, c->vcount, c->rho,
+                                             c->fin, c->nbr, c->tasks_b, pi + b,
+                                             pi + 2 * kPipeK + b, pi + 4 * kPipeK + b, vr));
+            if (b >= kPipeGathered) continue;
+            if (b == 0) SPHGB_CUDA(cudaStreamWaitEvent(st, e_vel, 0));
+            SPHGB_CUDA(launch_gather_vel_tasks(L, c->pidB, c->tasks_b, pi + b, pi + 4 * kPipeK + b,
+                                               c->vstart, c->vcount, sv, c->rho, c->velB, c->fin));
+        }
+        return SPHGB_OK;
+    };
+    // two buckets keep the GPU busy until the host knows the dependencies
+    rc = density_through(1);
+    if (rc) return rc;
     c->nbr_valid = true;
     // the slot counts and the dependencies are needed on the host to launch
     // and order the force buckets
@@ -1678,17 +1677,6 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
     const int32_t* h_slots = c->h_pipe + 5 * kPipeK;
     const int32_t* h_soff = c->h_pipe + 7 * kPipeK;
     const int32_t* h_dl = c->h_pipe + 8 * kPipeK;
-    int gathered = 0;   // buckets whose velocities are in slot order, as seen from st3
-    auto gather_through = [&](int last) -> int {
-        for (; gathered <= last; ++gathered) {
-            SPHGB_CUDA(cudaStreamWaitEvent(st3, e_bucket[gathered], 0));
-            if (gathered < kPipeGathered)
-                SPHGB_CUDA(launch_gather_vel_tasks(L3, c->pidB, c->tasks_b, pi + gathered,
-                                                   pi + 4 * kPipeK + gathered, c->vstart,
-                                                   c->vcount, sv, c->rho, c->velB, c->fin));
-        }
-        return SPHGB_OK;
-    };
     // range r downloads once force bucket max(r, dl[r]) is done (each force
     // bucket writes the FP64 rows of its particles)
     int next_r = 0;
@@ -1709,7 +1697,7 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
     };
     size_t listed = 0;
     for (int b = 0; b < kPipeK; ++b) {
-        rc = gather_through(std::min(std::max(h_dep[b], b), kPipeK - 1));
+        rc = density_through(std::min(std::max(h_dep[b], b), kPipeK - 1));
         if (rc) return rc;
         if (h_slots[b] < 0 || h_soff[b] < 0 || (size_t)h_soff[b] + h_slots[b] > N)
             return fail(SPHGB_ERR_STATE, "pipelined step: bucket slot counts out of range");
@@ -1720,24 +1708,21 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
         range.pos = sp;
         range.vel = sv;
         range.rho = sr;
-        rc = enqueue_forces(c, L3, &range, b);
+        rc = enqueue_forces(c, L, &range, b);
         if (rc) return rc;
-        SPHGB_CUDA(cudaEventRecord(e_range[b], st3));
+        SPHGB_CUDA(cudaEventRecord(e_range[b], st));
         rc = download_through(b);
         if (rc) return rc;
     }
     if (next_r != kPipeK) return fail(SPHGB_ERR_STATE, "pipelined step: range left undownloaded");
-    // every bucket gathered (the slot-order velocities are complete), then
-    // the checks and the step counter
-    rc = gather_through(kPipeK - 1);
+    rc = density_through(kPipeK - 1);       // all there already
     if (rc) return rc;
-    rc = enqueue_checks(c, st3);
+    rc = enqueue_checks(c, st);
     if (rc) return rc;
-    k_step_counter<<<blocks(c->n_scenes, 128), 128, 0, st3>>>(c->scene_step, c->n_scenes,
-                                                                c->step_limit);
+    k_step_counter<<<blocks(c->n_scenes, 128), 128, 0, st>>>(c->scene_step, c->n_scenes,
+                                                               c->step_limit);
     SPHGB_CUDA(cudaGetLastError());
     SPHGB_CUDA(cudaStreamSynchronize(st4));
-    SPHGB_CUDA(cudaStreamSynchronize(st3));
     SPHGB_CUDA(cudaStreamSynchronize(st));
     // every slot was in exactly one bucket
     if (listed != N) return fail(SPHGB_ERR_STATE, "pipelined step: buckets missed particles");
@@ -2045,8 +2030,7 @@ int sphgb_compute_next_state_host(SphgbCtx* ctx, const double* h_pos, const doub
     if (rc && ctx) {
         // a failed call returns only once nothing it enqueued still runs: no
         // copy into the caller's host buffers outlives the call
-        for (cudaStream_t s : {ctx->host_stream, ctx->host_stream2, ctx->host_stream3,
-                               ctx->host_stream4})
+        for (cudaStream_t s : {ctx->host_stream, ctx->host_stream2, ctx->host_stream4})
             if (s) cudaStreamSynchronize(s);
     }
     return rc;

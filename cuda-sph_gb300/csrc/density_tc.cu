@@ -370,7 +370,8 @@ __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uin
 
 // kLayout: 0 every scene's voxel table row-major, 1 every one tiled, 2 per scene.
 // Task t is at tasks[t * dir].  kUncapped: some scene's cap is beyond kListCap.
-template <int kLayout, bool kUncapped>
+// kGather: the task's velocities too, from FP64 rows (vrows).
+template <int kLayout, bool kUncapped, bool kGather>
 __global__ void __launch_bounds__(kTcWarps * 32, 6)
 k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
              int n_scenes, int n, const float4* __restrict__ pos,
@@ -378,7 +379,8 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
              const int32_t* __restrict__ vcount, float* __restrict__ rho,
              float4* __restrict__ fin, NbrList nbr,
              const int2* __restrict__ tasks, int dir, const int32_t* __restrict__ task_count,
-             int32_t* __restrict__ task_next) {
+             int32_t* __restrict__ task_next, const int32_t* __restrict__ task_offset,
+             VelRows vrows) {
     __shared__ TcShared sh[kTcWarps];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -386,6 +388,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const unsigned lt = (1u << lane) - 1u;
     int n_tasks = *grid_wait(task_count);
     if (nbr.veto && *after_wait(nbr.veto)) n_tasks = 0;
+    if (task_offset) tasks += *after_wait(task_offset);   // one bucket of a bucketed task list
     // A warp's first task is its own number; each later one comes from a
     // counter (the cost of a task varies with its voxel's neighbourhood, and a
     // fixed share per warp left warps idle at the end of the pass, 15 % of its
@@ -595,7 +598,14 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             if (home) {
                 const float r = (acc.s * sc.w_const) * sc.mass;
                 if (rho) rho[s] = r;
-                if (fin) write_force_inputs(s, pi, sc, vel, r, fin);
+                if (kGather) {
+                    const float4 v = vel_row(vrows, s, pbegin, n_scenes);
+                    vrows.vel_out[s] = v;
+                    stg256(fin + 2 * s, force_record_a(pi, sc, r),
+                           make_float4(v.x, v.y, v.z, 1.0f / r));
+                } else if (fin) {
+                    write_force_inputs(s, pi, sc, vel, r, fin);
+                }
                 if (nbr.count) nbr.count[s] = over ? -1 : others;
             }
         }
@@ -609,21 +619,24 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
 cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
                               float4* fin, NbrList nbr, const int2* tasks, int dir,
-                              const int32_t* task_count, int32_t* task_next, bool uncapped) {
+                              const int32_t* task_count, int32_t* task_next, bool uncapped,
+                              const int32_t* task_offset, VelRows vrows) {
     if (L.n == 0) return cudaSuccess;
     // persistent grid: up to 6 blocks of 4 warps per SM (shared memory), warps
     // take tasks in turn; small scenes get about a warp per task, so that the
     // tasks spread over the SMs (a task's latency is most of their pass)
     const int blocks = std::min((L.n + 8 * kTcWarps - 1) / (8 * kTcWarps), device_sm_count() * 6);
-    auto kernel = uncapped ? (L.layout == 1   ? k_density_tc<1, true>
-                              : L.layout == 2 ? k_density_tc<2, true>
-                                              : k_density_tc<0, true>)
-                           : (L.layout == 1   ? k_density_tc<1, false>
-                              : L.layout == 2 ? k_density_tc<2, false>
-                                              : k_density_tc<0, false>);
+    // the velocity gather is for one capped scene (the pipelined host order)
+    auto kernel = vrows.vel64 ? (L.layout == 1 ? k_density_tc<1, false, true> : k_density_tc<0, false, true>)
+                  : uncapped  ? (L.layout == 1   ? k_density_tc<1, true, false>
+                                 : L.layout == 2 ? k_density_tc<2, true, false>
+                                                 : k_density_tc<0, true, false>)
+                              : (L.layout == 1   ? k_density_tc<1, false, false>
+                                 : L.layout == 2 ? k_density_tc<2, false, false>
+                                                 : k_density_tc<0, false, false>);
     return launch_chained(kernel, blocks, kTcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
                           L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, dir, task_count,
-                          task_next);
+                          task_next, task_offset, vrows);
 }
 
 }  // namespace sphgb

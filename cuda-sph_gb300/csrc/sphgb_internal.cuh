@@ -599,6 +599,14 @@ struct VelRows {
     float4* vel_out = nullptr;       // slot order
 };
 
+// slot s's velocity from the FP64 rows (VelRows)
+__device__ __forceinline__ float4 vel_row(const VelRows& vr, int s,
+                                          const int32_t* __restrict__ pbegin, int n_scenes) {
+    const double* r =
+        vr.vel64 + 3 * (size_t)(__ldg(pbegin + scene_of(s, pbegin, n_scenes)) + __ldg(vr.pid + s));
+    return make_float4((float)__ldg(r), (float)__ldg(r + 1), (float)__ldg(r + 2), 0.0f);
+}
+
 struct PidRange {
     const int32_t* slot_of = nullptr;
     int i0 = 0, i1 = 0;
@@ -737,7 +745,8 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
 cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
                               float4* fin, NbrList nbr, const int2* tasks, int dir,
-                              const int32_t* task_count, int32_t* task_next, bool uncapped);
+                              const int32_t* task_count, int32_t* task_next, bool uncapped,
+                              const int32_t* task_offset = nullptr, VelRows vrows = VelRows{});
 // k_gather_vel over the slots of a bucket of density tasks
 cudaError_t launch_gather_vel_tasks(const Launch& L, const int32_t* pid, const int2* tasks,
                                     const int32_t* task_count, const int32_t* task_offset,

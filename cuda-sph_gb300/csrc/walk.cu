@@ -240,14 +240,6 @@ __device__ __forceinline__ void wc_candidates(WcShared& S, int& cnt, bool home, 
     }
 }
 
-// slot s's velocity from the FP64 rows (VelRows)
-__device__ __forceinline__ float4 vel_row(const VelRows& vr, int s,
-                                          const int32_t* __restrict__ pbegin, int n_scenes) {
-    const double* r =
-        vr.vel64 + 3 * (size_t)(__ldg(pbegin + scene_of(s, pbegin, n_scenes)) + __ldg(vr.pid + s));
-    return make_float4((float)__ldg(r), (float)__ldg(r + 1), (float)__ldg(r + 2), 0.0f);
-}
-
 // kLayout: 0 every scene's voxel table row-major, 1 every one tiled, 2 per scene.
 // kGather: the task's velocities too, from FP64 rows (vrows).
 template <int kLayout, bool kGather>

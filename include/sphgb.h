@@ -182,9 +182,10 @@ int sphgb_ctx_step_profiled(SphgbCtx* ctx, int n_steps, void* stream, float* h_s
  * abstract_sph_strategy.py:31-46, including its host<->device copies at
  * :65-74 and :77-84).  Context must hold exactly one scene.  Host buffers may
  * be pageable or page-locked (page-locked copies faster, and only they let
- * the copies overlap the step); they are copied through device staging
- * buffers.  A call that fails returns only after every copy it started has
- * finished. */
+ * the copies overlap the step).  They are copied through device staging
+ * buffers, or, for small scenes in slot order, read and written by the kernels
+ * themselves where the GPU reaches them.  A call that fails returns only after
+ * every copy and kernel it started has finished. */
 int sphgb_compute_next_state_host(SphgbCtx* ctx, const double* h_pos, const double* h_vel,
                                   double* h_pos_out, double* h_vel_out, double* h_rho_out);
 /* Order in which sphgb_compute_next_state_host runs its force pass (results
@@ -192,7 +193,7 @@ int sphgb_compute_next_state_host(SphgbCtx* ctx, const double* h_pos, const doub
  * state is downloaded whole.  SPHGB_HOST_ORDER_PARTICLE: original particle
  * order in ranges, each range's rows downloaded while the next range is
  * computed; faster when nearby particle ids are nearby in space, slower when
- * they are scattered.  SPHGB_HOST_ORDER_PIPELINED: the density pass in 16
+ * they are scattered.  SPHGB_HOST_ORDER_PIPELINED: the density pass in
  * buckets of tasks by the particle-id range of their first particle, the
  * force pass over each bucket's slots once every bucket its particles'
  * neighbours fall in is done, and each range's rows downloaded as soon as
