@@ -120,6 +120,7 @@ struct SphgbCtx {
     int v_total_ref = 0;       // reference layout
     int layout = 0;            // step layout: 0 all row-major, 1 all tiled, 2 mixed
     bool any_pipe = false;
+    bool pairs = false;        // density tasks of two voxels (TaskLists)
     bool uncapped = false;     // some scene's cap is beyond kListCap
     std::vector<SceneDev> h_scenes;
     std::vector<int32_t> h_pbegin;
@@ -265,6 +266,11 @@ struct SphgbCtx {
             t.tc_count = big_count + kTcCounter;
             t.tc_max = kTcVoxel;
         }
+        // With fewer particles than lanes at work every voxel has a warp of its own
+        // at once, and a pair takes longer (8,192 particles: step 27.3 us without,
+        // 27.5 with pairs; 15,294 in 6 boxes: 39.0 -> 34.2).
+        if (pairs && density_variant == SPHGB_DENSITY_WARP)
+            t.pair_max = n > 64 * device_sm_count() ? kTaskRun : 0;
         return t;
     }
 
@@ -1034,6 +1040,21 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
         if (d.mode == SPHGB_MODE_PIPE) any_pipe = true;
     }
     hp[n_scenes] = (int32_t)n_tot;
+    // Density tasks of two voxels (TaskLists): every scene tiled, its table at
+    // whole tiles, and the voxels that a pair's particles walk in excess out of
+    // their reach.
+    bool pairs = n_tot > 0;
+    for (const SceneDev& d : hs) pairs = pairs && d.tiled && d.vs[2] >= d.h;
+    int64_t v_tiles = 0;
+    for (const SceneDev& d : hs) v_tiles += d.v_count + 64;
+    pairs = pairs && v_tiles < (int64_t)0x7fffffff;
+    if (pairs) {
+        v_tot = 0;
+        for (SceneDev& d : hs) {
+            d.v_begin = (int32_t)v_tot;
+            v_tot += d.v_count + 64;
+        }
+    }
     std::vector<ConsChunk> chunks;
     for (int i = 0; i < n_scenes; ++i) {
         const SceneDev& d = hs[i];
@@ -1089,6 +1110,7 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
     int n_tiled = 0;
     for (const SceneDev& d : c->h_scenes) n_tiled += d.tiled;
     c->layout = n_tiled == 0 ? 0 : (n_tiled == n_scenes ? 1 : 2);
+    c->pairs = pairs;
     c->big_count = c->counts;
     c->scan_status = reinterpret_cast<unsigned long long*>(c->counts + kCountersPad);
     c->vcount = c->counts + head;

@@ -12,8 +12,9 @@ namespace sphgb {
 namespace {
 
 // Warp-cooperative density pass of the step.  One warp per task: up to
-// kTaskRun particles ("homes") of one voxel (tasks listed by the rank-gather).
-// The 27 walk voxels of that voxel are laid end to end in walk order and taken
+// kTaskRun particles ("homes") of one voxel, or of two that are neighbours in z
+// (tasks listed by the rank-gather, see TaskLists).  The 27 walk voxels of that
+// voxel, or the 36 of the two, are laid end to end in walk order and taken
 // in chunks of kTcChunk candidates.  Per chunk:
 //
 // Phase 1 decides every (home, candidate) pair into one bit, 32 candidates (a
@@ -39,9 +40,9 @@ namespace {
 // What bounds it: instruction issue (69 % of the issue slots with 24 warps per
 // SM) beside shared memory (67 % of its wavefronts).  A 4,194,304-particle box
 // at 11 particles per voxel: 1.171 ms with the ballots and per-home ranking of
-// k_density_wc, 1.003 ms here, 2765 against 2090 warp instructions per task of
-// 10 homes (390 to set up, 100 per group of candidates for all homes, 800 in
-// phase 2).  262,144 particles: 88 -> 73 us.  Measured and not kept: 32 warps per
+// k_density_wc, 0.948 ms here, 2765 against 2000 warp instructions per task of
+// 10 homes (400 to set up, 100 per group of candidates for all homes, 760 in
+// phase 2).  262,144 particles: 88 -> 71 us.  Measured and not kept: 32 warps per
 // SM at 64 registers (1.09 ms: spills, 20 % more instructions), 16-bit list
 // entries, one lane per (home, word) extracting the bits into lists and one
 // lane per list entry for the terms (1.29 ms: dense words make the extraction
@@ -55,13 +56,14 @@ constexpr int kTcWords = kTcChunk / 32;
 constexpr int kTcCullMin = 640;  // walks longer than this pass over unreachable batches
 constexpr int kTcBallot = 4;     // tasks of at most this many homes test with ballots
 // Bound on |computed - exact| of (d^2 - h^2) / vs^2 for candidates of |u|^2 <=
-// kTcFar, homes of |u|^2 <= 1 and (h / vs)^2 <= kTcH2 (others are decided by
-// ballots): every partial sum is below 8 + 2 sqrt(8) + 2 < 16.  The FP32
-// rounding of u and |u|^2 gives 2^-17.6, the FP16 pairs 2^-17.6 over the
-// products and |u|^2, 17 accumulations truncated at 2^-20 each 2^-15.9:
-// 2^-15 = 3e-5 together.
+// kTcFar, homes of |u|^2 <= kTcHome and (h / vs)^2 <= kTcH2 (others are decided
+// by ballots): every partial sum is below 9 + 2 sqrt(9 * 1.6) + 2 < 32.  The FP32
+// rounding of u and |u|^2 gives 2^-17.4, the FP16 pairs 2^-17.4 over the products
+// and |u|^2, 17 accumulations truncated at 2^-19 each 2^-14.9: 2^-14.4 = 5e-5
+// together.
 constexpr float kTcTol = 1.0e-4f;
-constexpr float kTcFar = 8.0f;   // 3 * 1.5^2 and room: |u|^2 inside the 27 voxels
+constexpr float kTcFar = 9.0f;    // |u|^2 within the walk: 3 * 1.5^2, pairs 2 * 1.5^2 + 2^2
+constexpr float kTcHome = 1.6f;   // 3 * 0.5^2, pairs 2 * 0.5^2 + 1
 constexpr float kTcH2 = 2.0f;
 static_assert(kTcChunk % kTcBatch == 0, "a chunk is whole batches");
 static_assert(kTaskRun == 16 && kTaskRun <= kSumSplit, "16 rows per mma, two lanes per home");
@@ -73,7 +75,9 @@ struct alignas(16) TcShared {
     uint4 feat[kTcBatch];              // FP16 features of a batch, in ldmatrix order
     int32_t list[kTaskRun][kTcRow];    // neighbour slots in walk order
     uint32_t mask[kTaskRun][kTcMaskRow];   // accepted candidates: word q >> 5, q & 31 from the top bit
-    int32_t off[27];   // first slot - first walk index of each non-empty walk voxel, by rank
+    uint32_t seg[kTcWords];       // chunk's places where a walk voxel starts, bit q & 31 of word q >> 5
+    uint32_t reach1[16];          // see TcWalk
+    int32_t off[36];              // first slot - first walk index of each non-empty walk voxel, by rank
 };
 
 __device__ __forceinline__ uint32_t half2_bits(float lo, float hi) {
@@ -139,16 +143,34 @@ __device__ __forceinline__ unsigned group_mask(const float4& ph, const float4& p
     return __brev(__ballot_sync(0xffffffffu, acc));
 }
 
+// A task's walk as one lane holds it: lane l < 18 has the column l / 2 of the
+// walk (x and y neighbours, in walk order) and two of its voxels in z, with
+// the walk indices where they start and end.  reach0 and S.reach1 of home lane &
+// 15 (long walks): bit l set when lane l's first or second voxel may hold a
+// particle within h of it.
+struct TcWalk {
+    int p0, p1, end;
+    unsigned reach0;
+    __device__ __forceinline__ bool has0() const { return p1 > p0; }
+    __device__ __forceinline__ bool has1() const { return end > p1; }
+    // Sets S.seg's bits for the chunk at c0.  Candidate q of the walk lies in the
+    // last non-empty walk voxel that starts at or before it, found by counting
+    // the bits.
+    __device__ __forceinline__ void mark(TcShared& S, int c0) const {
+        const unsigned a = p0 - c0, b = p1 - c0;
+        if (has0() && a < kTcChunk) atomicOr(&S.seg[a >> 5], 1u << (a & 31));
+        if (has1() && b < kTcChunk) atomicOr(&S.seg[b >> 5], 1u << (b & 31));
+    }
+};
+
 // Phase 1 for the candidates [c0, c1) of one task: writes S.cand and S.mask
 // and returns the number of groups decided; T receives each home's accepted
 // candidates (lanes i and 16 + i: home i), and (gh, Th) the last word with at
 // most kSumSplit accepted candidates of the home before it, and how many of
 // them are in the chunk.  Stops early once every home has `cap` (cnt: accepted
-// before this chunk).  Lane k < 27 holds walk voxel k's first walk index Pk and
-// member count ck; cull: see reach_mask.
+// before this chunk).  cull: batches that no home reaches are passed over.
 __device__ __forceinline__ int tc_decide(TcShared& S, int& T, int& gh, int& Th, int cnt, int c_t,
-                                         int cap, int c0, int c1, int Pk, int ck, bool nzk,
-                                         bool cull, unsigned reach,
+                                         int cap, int c0, int c1, const TcWalk& W, bool cull,
                                          const uint32_t (&A)[4], const float (&C)[4], bool ballots,
                                          const TcFrame& F, const float4& pi,
                                          const float4* __restrict__ pos, int n, const SceneDev& sc) {
@@ -156,6 +178,17 @@ __device__ __forceinline__ int tc_decide(TcShared& S, int& T, int& gh, int& Th, 
     const int lane = threadIdx.x & 31;
     const int ih = lane & 15;
     const unsigned le = (2u << lane) - 1u;      // bits 0..lane
+    // rank: the last non-empty walk voxel that starts before the group, taking bit
+    // 0 of the chunk's first word for a start
+    int rank = -1;
+    if (c0 > 0) {
+        if (lane < kTcWords) S.seg[lane] = lane == 0 ? 1u : 0u;
+        rank += __popc(__ballot_sync(full, W.has0() && W.p0 <= c0)) +
+                __popc(__ballot_sync(full, W.has1() && W.p1 <= c0)) - 1;
+        __syncwarp();
+        W.mark(S, c0);
+        __syncwarp();
+    }
     // Candidate l of a group is column n = 2 (l / 8) + l % 2 of mma t =
     // (l / 2) % 4, so that lane 4 r + q ends up with the decisions of home r
     // (and r + 8) on candidates 8 q .. 8 q + 7, byte 3 - q of the mask word.  The
@@ -174,37 +207,30 @@ __device__ __forceinline__ int tc_decide(TcShared& S, int& T, int& gh, int& Th, 
         if (cull) {
             // walk voxels overlapping this batch: skipped when no home below
             // the cap reaches one (those voxels hold no accepted candidate)
-            const unsigned span = __ballot_sync(full, nzk && Pk < b0 + kTcBatch && Pk + ck > b0);
-            if (!__any_sync(full, ih < c_t && cnt + T < cap && (reach & span) != 0u)) {
+            const unsigned s0 = __ballot_sync(full, W.has0() && W.p0 < b0 + kTcBatch && W.p1 > b0);
+            const unsigned s1 = __ballot_sync(full, W.has1() && W.p1 < b0 + kTcBatch && W.end > b0);
+            if (!__any_sync(full, ih < c_t && cnt + T < cap &&
+                                      ((W.reach0 & s0) | (S.reach1[ih] & s1)) != 0u)) {
 #pragma unroll
                 for (int u = 0; u < kTcGroups; ++u) {
                     if (lane < kTaskRun) S.mask[ih][G + u] = 0u;
                     if (cnt + T <= kSumSplit) { gh = G + u; Th = T; }
+                    rank += __popc(S.seg[G + u]);
                 }
                 __syncwarp();
                 continue;
             }
         }
-        // Batch candidates q = b0 + 32 u + lane.  Bw[u] bit l: a non-empty
-        // walk voxel starts at q = b0 + 32 u + l (l >= 1 when u = 0); the
-        // rank of the voxel holding q is the number of non-empty voxels
-        // starting at or before b0, minus one, plus the set bits up to q.
-        const int pk = Pk - b0;
-        unsigned Bw[kTcGroups];
-#pragma unroll
-        for (int u = 0; u < kTcGroups; ++u)
-            Bw[u] = __reduce_or_sync(
-                full, (nzk && pk >= 1 && (pk >> 5) == u) ? (1u << (pk & 31)) : 0u);
-        int rank = __popc(__ballot_sync(full, nzk && pk <= 0)) - 1;
         // Past the end of the walk (the last batch) some particle stands in,
         // and its bits are cut off below.
         float4 pj[kTcGroups];
 #pragma unroll
         for (int u = 0; u < kTcGroups; ++u) {
-            const int sj = min(b0 + 32 * u + lane + S.off[rank + __popc(Bw[u] & le)], n - 1);
+            const unsigned starts = S.seg[G + u];
+            const int sj = min(b0 + 32 * u + lane + S.off[rank + __popc(starts & le)], n - 1);
             pj[u] = __ldg(pos + sj);
             pj[u].w = __int_as_float(sj);
-            rank += __popc(Bw[u]);
+            rank += __popc(starts);
         }
         // the bits of group u that are candidates
         auto valid = [&](int u) {
@@ -386,6 +412,8 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     const int lane = threadIdx.x & 31;
     TcShared& S = sh[threadIdx.x >> 5];
     const unsigned lt = (1u << lane) - 1u;
+    if (lane < kTcWords) S.seg[lane] = 0u;
+    __syncwarp();
     int n_tasks = *grid_wait(task_count);
     if (nbr.veto && *after_wait(nbr.veto)) n_tasks = 0;
     if (task_offset) tasks += *after_wait(task_offset);   // one bucket of a bucketed task list
@@ -400,19 +428,13 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         if (t >= n_tasks) break;
         const int2 task = after_wait(tasks)[t * dir];
         if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
-        const int vid = task.x, d0 = task.y;
+        // a pair task (see TaskLists) has its first voxel's index complemented
+        const bool pair = kLayout == 1 && !kGather && task.x < 0;
+        const int vid = pair ? ~task.x : task.x, d0 = task.y;
         const SceneDev& sc = scenes[scene_of_warp(d0, pbegin, n_scenes)];
-        const int vst = __ldg(vstart + vid), vc = __ldg(vcount + vid);
-        const int c_t = min(kTaskRun, vst + vc - d0);
-        const int s = d0 + lane;
-        const bool home = lane < c_t;
         const int local = vid - sc.v_begin;
         const int cap = sc.cap;
-        // lanes i and 16 + i: home i
-        const int ih = lane & 15;
-        const bool upper = lane >= 16;
-        const float4 pi = ih < c_t ? __ldg(pos + d0 + ih) : make_float4(0.f, 0.f, 0.f, 0.f);
-        // the 27 walk voxels (voxel_kernels.py:46-61 order), from the table coords
+        // the walk voxels (voxel_kernels.py:46-61 order), from the table coords
         const int tiled = kLayout == 2 ? sc.tiled : kLayout;
         // index -> coordinates with the scene's multiply-shift reciprocals
         const Udiv q0{sc.div_m[0], sc.div_s[0]}, q1{sc.div_m[1], sc.div_s[1]};
@@ -429,17 +451,44 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             vy = r0 - r1 * sc.dims[1];
             vz = r1;
         }
-        int ck = 0, stk = 0, idk = -1;
-        if (lane < 27) {
+        // 9 columns of 3 voxels in z, or of 4 for a pair: each home's own walk is
+        // in order in them, and the voxel that is not in it lies a whole voxel
+        // side away, so that its particles are beyond h
+        TcWalk W{0, 0, 0, 0u};
+        int wc0, wc1, st0, st1, id0, id1;
+        {
+            const int col = lane >> 1, half = lane & 1;
+            const int nx = vx + col / 3 - 1, ny = vy + col % 3 - 1, nz = vz - 1 + 2 * half;
             const int w0 = sc.wdims[0], w1 = sc.wdims[1], w2 = sc.wdims[2];
-            const int nx = vx + lane / 9 - 1, ny = vy + (lane / 3) % 3 - 1, nz = vz + lane % 3 - 1;
-            if (nx >= 0 && nx < w0 && ny >= 0 && ny < w1 && nz >= 0 && nz < w2) {
-                idk = sc.v_begin + voxel_index(nx, ny, nz, tiled, w0, w1, sc.nt0, sc.nt1);
-                ck = __ldg(vcount + idk);
-                stk = __ldg(vstart + idk);
-            }
+            const bool in = lane < 18 && nx >= 0 && nx < w0 && ny >= 0 && ny < w1;
+            const bool in0 = in && nz >= 0 && nz < w2, in1 = in && (half == 0 || pair) && nz + 1 < w2;
+            id0 = in0 ? sc.v_begin + voxel_index(nx, ny, nz, tiled, w0, w1, sc.nt0, sc.nt1) : vid;
+            id1 = in1 ? sc.v_begin + voxel_index(nx, ny, nz + 1, tiled, w0, w1, sc.nt0, sc.nt1) : vid;
+            wc0 = __ldg(vcount + id0);
+            wc1 = __ldg(vcount + id1);
+            st0 = __ldg(vstart + id0);
+            st1 = __ldg(vstart + id1);
+            wc0 = in0 ? wc0 : 0;
+            wc1 = in1 ? wc1 : 0;
         }
-        int incl = ck;
+        // lanes i and 16 + i: home i, at slot s (loaded beside the counts that say
+        // how many there are)
+        const int ih = lane & 15;
+        int s = d0 + ih;
+        float4 pi = __ldg(pos + min(s, n - 1));
+        // the task's particles: a run of its voxel, or all of the pair's two (the
+        // second voxel is the first one of lane 9)
+        const int vst = __ldg(vstart + vid), vc = __ldg(vcount + vid);
+        const int st_b = __shfl_sync(full, st0, 9), c_b = __shfl_sync(full, wc0, 9);
+        const int c_a = min(kTaskRun, vst + vc - d0);
+        const int c_t = pair ? c_a + c_b : c_a;
+        const bool upper = lane >= 16, home = lane < c_t;
+        if (ih >= c_a) {
+            s = st_b + ih - c_a;
+            pi = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ih < c_t) pi = __ldg(pos + s);
+        }
+        int incl = wc0 + wc1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(full, incl, o);
@@ -447,24 +496,37 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         }
         // candidates in the whole walk; none for the overflow entry, whose
         // particles (non-finite positions) have no neighbours
-        const int M = local == sc.v_count ? 0 : __shfl_sync(full, incl, 26);
+        const int M = local == sc.v_count ? 0 : __shfl_sync(full, incl, 17);
         // Candidate q (walk order) lies in the non-empty walk voxel with the
-        // largest first index P_k <= q; its slot is q + (start_k - P_k).  Lane
-        // k keeps P_k; S.off holds start_k - P_k by rank among the non-empty
-        // walk voxels.
-        const int Pk = incl - ck;
-        const bool nzk = lane < 27 && ck > 0;
-        const unsigned NZ = __ballot_sync(full, nzk);
-        if (nzk) S.off[__popc(NZ & lt)] = stk - Pk;
-        // the walk voxel that is the task's own (a truncated walk may miss it)
-        // gives the homes' own walk indices
-        const unsigned own = __ballot_sync(full, nzk && idk == vid);
-        const int P_own = __shfl_sync(full, Pk, own ? __ffs(own) - 1 : 0);
-        const int q_self = own ? P_own + (d0 - vst) + ih : -1;
+        // largest first index P <= q; its slot is q + (start - P).  S.off holds
+        // start - P by rank among the non-empty walk voxels.
+        W.end = incl;
+        W.p1 = incl - wc1;
+        W.p0 = W.p1 - wc0;
+        W.mark(S, 0);       // cleared before the task
+        {
+            const unsigned N0 = __ballot_sync(full, wc0 > 0), N1 = __ballot_sync(full, wc1 > 0);
+            const int k = __popc(N0 & lt) + __popc(N1 & lt);
+            if (wc0 > 0) S.off[k] = st0 - W.p0;
+            if (wc1 > 0) S.off[k + (wc0 > 0)] = st1 - W.p1;
+        }
+        // the homes' own walk indices: the task's voxel is the second one of lane 8
+        // (of another one, or of none, in a truncated walk, which no tiled scene has)
+        int q_self;
+        if (kLayout == 1) {
+            const int P = __shfl_sync(full, W.p1, 8), Pb = __shfl_sync(full, W.p0, 9);
+            q_self = ih < c_a ? P + (d0 - vst) + ih : Pb + ih - c_a;
+        } else {
+            const unsigned own0 = __ballot_sync(full, wc0 > 0 && id0 == vid);
+            const unsigned own1 = __ballot_sync(full, wc1 > 0 && id1 == vid);
+            const int P0 = __shfl_sync(full, W.p0, own0 ? __ffs(own0) - 1 : 0);
+            const int P1 = __shfl_sync(full, W.p1, own1 ? __ffs(own1) - 1 : 0);
+            q_self = own0 | own1 ? (own1 ? P1 : P0) + (d0 - vst) + ih : -1;
+        }
         __syncwarp();
         // the homes' side of the contraction (rows lane / 4 and lane / 4 + 8)
         const TcFrame F{((float)vx + 0.5f) * sc.vs[0], ((float)vy + 0.5f) * sc.vs[1],
-                        ((float)vz + 0.5f) * sc.vs[2], sc.u_scale};
+                        ((float)vz + (pair ? 1.0f : 0.5f)) * sc.vs[2], sc.u_scale};
         uint32_t A[4] = {0u, 0u, 0u, 0u};
         float C0[4] = {1.0f, 1.0f, 1.0f, 1.0f};      // rows without a home accept nothing
         bool ballots = c_t <= kTcBallot || !(sc.u_h2 <= kTcH2);
@@ -488,7 +550,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
                 }
             }
             // a home outside its voxel (clamped coordinates)
-            ballots = __any_sync(full, ih < c_t && !(c <= 1.0f));
+            ballots = __any_sync(full, ih < c_t && !(c <= kTcHome));
         }
         // through an mma of zeros, into the four consecutive registers that the
         // others read in place (as plain values they were copied for each)
@@ -500,8 +562,20 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         // Long walks: each home's 27-bit mask of the walk voxels within h of it
         // (box distance, the walk's culling test), so that batches in voxels
         // that no home can reach are passed over.
-        const bool cull = !sc.walk_trunc && M > kTcCullMin;
-        const unsigned reach = cull ? reach_mask(pi, vx, vy, vz, sc) : 0u;
+        const bool cull = !sc.walk_trunc && !pair && M > kTcCullMin;
+        if (cull) {
+            // walk voxel 3 col + z is lane 2 col's first (z 0), second (1) or lane 2 col + 1's first (2)
+            const unsigned reach = reach_mask(pi, vx, vy, vz, sc);
+            unsigned reach1 = 0u;
+#pragma unroll
+            for (int col = 0; col < 9; ++col) {
+                W.reach0 |= (reach >> (3 * col) & 1u) << (2 * col) |
+                            (reach >> (3 * col + 2) & 1u) << (2 * col + 1);
+                reach1 |= (reach >> (3 * col + 1) & 1u) << (2 * col);
+            }
+            if (!upper) S.reach1[ih] = reach1;
+            __syncwarp();
+        }
         // the row may not hold every neighbour
         const bool uncapped = kUncapped && cap > kListCap;
         const float inv_h2 = sc.inv_h2;
@@ -513,7 +587,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         for (int c0 = 0; c0 < M; c0 += kTcChunk) {
             const int c1 = min(M, c0 + kTcChunk);
             int T, gh, Th;
-            const int G = tc_decide(S, T, gh, Th, cnt, c_t, cap, c0, c1, Pk, ck, nzk, cull, reach, A, Cq, ballots, F, pi,
+            const int G = tc_decide(S, T, gh, Th, cnt, c_t, cap, c0, c1, W, cull, A, Cq, ballots, F, pi,
                                     pos, n, sc);
             if (uncapped && c0 == 0 && nbr.over) {
                 // room for the lists that will not fit their rows: of known
@@ -570,6 +644,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             if (!__any_sync(full, home && cnt < cap)) break;
         }
         __syncwarp();
+        if (lane < kTcWords) S.seg[lane] = 0u;      // for the next task
         if (kUncapped && home && others > kListCap) {
             S.list[ih][0] = unit >= 0 ? others : 0;
             S.list[ih][1] = (int)unit;
@@ -581,8 +656,9 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
 #pragma unroll
             for (int i0 = 0; i0 < kTaskRun; i0 += 4) {
                 const int i = i0 + (lane >> 3), k = 4 * (lane & 7);
+                const int si = __shfl_sync(full, s, i);
                 if (i < c_t)
-                    *reinterpret_cast<int4*>(nbr.idx + (size_t)(d0 + i) * kListCap + k) =
+                    *reinterpret_cast<int4*>(nbr.idx + (size_t)si * kListCap + k) =
                         *reinterpret_cast<const int4*>(&S.list[i][k]);
             }
         }

@@ -648,6 +648,8 @@ struct Launch {
     int layout = 0;             // voxel tables: 0 all row-major, 1 all tiled, 2 mixed
     cudaStream_t stream;
     bool chained = true;        // see launch_chained
+    int smem_share = 0;         // chained launches: preferred share of an SM's L1 for shared
+                                // memory, percent; 0: what the kernel itself needs
     // per-scene step limits and counters (device, n_scenes each); limits null:
     // no scene is frozen.  A frozen scene's particles keep their slots in the
     // sort, get no density task and are copied through by the force pass.
@@ -663,15 +665,17 @@ struct Launch {
 template <class... P, class... A>
 cudaError_t launch_chained(void (*kernel)(P...), int blocks, int threads, const Launch& L,
                            A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[1].val.sharedMemCarveout = (unsigned)L.smem_share;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = L.stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = L.chained ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = !L.chained ? 0 : L.smem_share > 0 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
@@ -702,12 +706,21 @@ constexpr int kTaskRun = 16;
 // tc_last (entry t at tc_last[-t]); the others to the list from `list` on.
 // Both share one array: there are no more tasks than particles.  list null:
 // no tasks.
+//
+// Pairs (contexts whose scenes are all tiled, with voxels at least h deep): two
+// voxels that are neighbours in z, 2k and 2k + 1, of at most pair_max <= kTaskRun
+// particles together are one task, (~first voxel, first slot).  Their table
+// indices differ in bit 4.  k_density_tc pays most of a task's cost per task,
+// not per particle, and two voxels' walks share half their voxels: 48 boxes of
+// 8 particles per voxel, 699,220 in all, 235 -> 146 us of density; a box of
+// 4,194,304 at 11 per voxel, where few pairs fit, 993 -> 948.
 struct TaskLists {
     int2* list = nullptr;
     int32_t* count = nullptr;
     int2* tc_last = nullptr;
     int32_t* tc_count = nullptr;
     int tc_max = 0;      // one list
+    int pair_max = 0;    // 0: none
 };
 // tmp_pid must be 16-byte aligned with 4 entries of room past n (the rank
 // count reads it in aligned quads).
