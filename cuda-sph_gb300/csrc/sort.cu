@@ -322,6 +322,8 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
     }
 }
 
+// kRows64: pipe scenes, with FP64 position rows to move too
+template <bool kRows64>
 __global__ void __launch_bounds__(512)
 k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict__ pid,
               const int32_t* __restrict__ tmp_pid, const int32_t* __restrict__ vstart,
@@ -339,7 +341,7 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
         pid_out[s] = pid[s];
         pos_out[s] = __ldg(pos + s);
         if (vel) vel_out[s] = __ldg(vel + s);
-        if (pos64) {
+        if (kRows64) {
             pos64_out[3 * s + 0] = pos64[3 * s + 0];
             pos64_out[3 * s + 1] = pos64[3 * s + 1];
             pos64_out[3 * s + 2] = pos64[3 * s + 2];
@@ -349,6 +351,15 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
     const int code = cell[s];
     const int vid = code < 0 ? ~code : code;
     const int p = pid[s];
+    // The chain from the cell to the rank is most of a small scene's pass: the
+    // rows are loaded beside it, and the ids two quads at a time (8,192 particles:
+    // step 27.1 -> 26.7 us, 699,220 in 48 boxes: pass 23.4 -> 22.7).  Not in pipe
+    // scenes, whose threads have the FP64 rows to move too (pass 33 -> 36 us).
+    float4 row = make_float4(0.f, 0.f, 0.f, 0.f), vrow = row;
+    if (!kRows64) {
+        row = __ldg(pos + s);
+        if (vel) vrow = __ldg(vel + s);
+    }
     const int st = __ldg(vstart + vid);
     const int c = __ldg(vcount + vid);
     int r = 0;
@@ -357,12 +368,18 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
     } else if (c <= big_voxel) {
         // the voxel's ids four per load from the aligned quad at or before st;
         // entries outside [st, st + c) are masked (tmp_pid is 16-byte aligned
-        // and padded by 4 entries, so the last quad stays inside it)
+        // and padded by 4 entries, so the last quad stays inside it; a second quad
+        // past the end is not loaded)
         const int e = st + c;
-        for (int k = st & ~3; k < e; k += 4) {
+#pragma unroll 1
+        for (int k = st & ~3; k < e; k += 8) {
             const int4 q = __ldg(reinterpret_cast<const int4*>(tmp_pid + k));
+            const int k2 = k + 4 < e ? k + 4 : k;
+            const int4 q2 = __ldg(reinterpret_cast<const int4*>(tmp_pid + k2));
             r += (k >= st && q.x < p) + (k + 1 >= st && k + 1 < e && q.y < p) +
                  (k + 2 >= st && k + 2 < e && q.z < p) + (k + 3 < e && q.w < p);
+            r += (k + 4 < e && q2.x < p) + (k + 5 < e && q2.y < p) + (k + 6 < e && q2.z < p) +
+                 (k + 7 < e && q2.w < p);
         }
     } else {                            // sorted by k_sort_big: lower bound of p
         int lo = 0, hi = c;
@@ -390,9 +407,13 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
             tasks.list[atomicAdd(tasks.count, 1)] = make_int2(first, d);
     }
     pid_out[d] = p;
-    pos_out[d] = __ldg(pos + s);
-    if (vel) vel_out[d] = __ldg(vel + s);   // null: velocities gathered later
-    if (pos64) {
+    if (kRows64) {
+        row = __ldg(pos + s);
+        if (vel) vrow = __ldg(vel + s);
+    }
+    pos_out[d] = row;
+    if (vel) vel_out[d] = vrow;             // null: velocities gathered later
+    if (kRows64) {
         pos64_out[3 * d + 0] = pos64[3 * s + 0];
         pos64_out[3 * d + 1] = pos64[3 * s + 1];
         pos64_out[3 * d + 2] = pos64[3 * s + 2];
@@ -448,14 +469,15 @@ cudaError_t launch_rank_gather(const Launch& L, const int32_t* cell, const int32
     // The density pass is chained to this one, its blocks fill the shared memory,
     // and an SM is not set up anew while it has blocks: this pass runs with the
     // density pass's set-up (17,280 particles: step 35.8 -> 34.5 us, 51,911: 49.9
-    // -> 48.9; the pass itself takes the same time).  A density pass that is not
-    // chained is as fast there but loses 1 to 3 us in a single step.
+    // -> 48.9).  A density pass that is not chained is as fast there but loses 1 to
+    // 3 us in a single step.  More particles than resident threads use what the
+    // blocks before left in L1 (4,194,304: pass 97 us, 120 with little L1).
     Launch next = L;
-    if (tasks.list) next.smem_share = 100;
-    return launch_chained(k_rank_gather, (L.n + b - 1) / b, b, next, L.n, cell, pid, tmp_pid,
-                          vstart, vcount, pos, vel, pos64, pos_out, vel_out, pid_out, pos64_out,
-                          tasks, L.big_voxel, slot, L.pbegin, L.n_scenes, L.step_limit,
-                          L.scene_step);
+    if (tasks.list && L.n <= 2048 * device_sm_count()) next.smem_share = 100;
+    return launch_chained(pos64 ? k_rank_gather<true> : k_rank_gather<false>, (L.n + b - 1) / b, b,
+                          next, L.n, cell, pid, tmp_pid, vstart, vcount, pos, vel, pos64, pos_out,
+                          vel_out, pid_out, pos64_out, tasks, L.big_voxel, slot, L.pbegin,
+                          L.n_scenes, L.step_limit, L.scene_step);
 }
 
 }  // namespace sphgb
