@@ -150,7 +150,7 @@ __device__ __forceinline__ int look_back(const int32_t* __restrict__ vcount, int
 
 __global__ void __launch_bounds__(kScanThreads)
 k_scan(const int32_t* __restrict__ vcount, int v_total, unsigned long long* status,
-       int32_t* __restrict__ vstart) {
+       int32_t* __restrict__ vstart, int4* __restrict__ next_counts, int next_quads) {
     __shared__ int s_before;
     const int tile = grid_wait((int)blockIdx.x);
     const int base = tile * kScanTile + threadIdx.x * kScanItems;
@@ -199,6 +199,9 @@ k_scan(const int32_t* __restrict__ vcount, int v_total, unsigned long long* stat
 #pragma unroll
         for (int i = 0; i < kScanItems; ++i) if (base + i < v_total) vstart[base + i] = out[i];
     }
+    // the next step's counters, status words and counts
+    for (int k = blockIdx.x * kScanThreads + threadIdx.x; k < next_quads; k += gridDim.x * kScanThreads)
+        next_counts[k] = make_int4(0, 0, 0, 0);
 }
 
 __global__ void __launch_bounds__(512)
@@ -435,9 +438,12 @@ cudaError_t launch_hash_count(const Launch& L, const float4* pos, int32_t* cell,
 }
 
 cudaError_t launch_scan(const Launch& L, const int32_t* vcount, int32_t* vstart,
-                        unsigned long long* status, int n_tiles) {
+                        unsigned long long* status, int n_tiles, int32_t* next_counts,
+                        size_t next_ints) {
     if (L.v_total == 0) return cudaSuccess;
-    return launch_chained(k_scan, n_tiles, kScanThreads, L, vcount, L.v_total, status, vstart);
+    return launch_chained(k_scan, n_tiles, kScanThreads, L, vcount, L.v_total, status, vstart,
+                          reinterpret_cast<int4*>(next_counts),
+                          next_counts ? (int)(next_ints / 4) : 0);
 }
 
 cudaError_t launch_scatter(const Launch& L, const int32_t* cell, const int32_t* slot,

@@ -685,9 +685,12 @@ cudaError_t launch_chained(void (*kernel)(P...), int blocks, int threads, const 
 // (the arrival order inside a voxel is dropped by the rank-gather).
 cudaError_t launch_hash_count(const Launch& L, const float4* pos, int32_t* cell, int32_t* slot,
                               int32_t* vcount, int i0 = 0, int i1 = -1);
-// status: scan_tiles(v_total) words, zero before the launch
+// status: scan_tiles(v_total) words, zero before the launch.  next_counts
+// (optional): a buffer that the pass clears, for the step after this one;
+// next_ints a multiple of 4, 16-byte aligned.
 cudaError_t launch_scan(const Launch& L, const int32_t* vcount, int32_t* vstart,
-                        unsigned long long* status, int n_tiles);
+                        unsigned long long* status, int n_tiles, int32_t* next_counts = nullptr,
+                        size_t next_ints = 0);
 int scan_tiles(int v_total);
 cudaError_t launch_scatter(const Launch& L, const int32_t* cell, const int32_t* slot,
                            const int32_t* pid, const int32_t* vstart, const int32_t* vcount,
