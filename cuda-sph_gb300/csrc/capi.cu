@@ -286,6 +286,7 @@ struct SphgbCtx {
         // With fewer particles than lanes at work every voxel has a warp of its own
         // at once, and a pair takes longer (8,192 particles: step 27.3 us without,
         // 27.5 with pairs; 15,294 in 6 boxes: 39.0 -> 34.2).
+        t.tc_next = density_variant == SPHGB_DENSITY_WARP && density_pass() == kPassTc;
         if (pairs && density_variant == SPHGB_DENSITY_WARP)
             t.pair_max = n > 64 * device_sm_count() ? kTaskRun : 0;
         return t;

@@ -472,14 +472,15 @@ cudaError_t launch_rank_gather(const Launch& L, const int32_t* cell, const int32
                                int32_t* pid_out, double* pos64_out, TaskLists tasks) {
     if (L.n == 0) return cudaSuccess;
     const int b = L.sort_block;
-    // The density pass is chained to this one, its blocks fill the shared memory,
-    // and an SM is not set up anew while it has blocks: this pass runs with the
-    // density pass's set-up (17,280 particles: step 35.8 -> 34.5 us, 51,911: 49.9
+    // k_density_tc is chained to this one, its blocks fill the shared memory, and an
+    // SM is not set up anew while it has blocks: this pass runs with the density
+    // pass's set-up (17,280 particles: step 35.8 -> 34.5 us, 51,911: 49.9
     // -> 48.9).  A density pass that is not chained is as fast there but loses 1 to
     // 3 us in a single step.  More particles than resident threads use what the
-    // blocks before left in L1 (4,194,304: pass 97 us, 120 with little L1).
+    // blocks before left in L1 (4,194,304: pass 97 us, 120 with little L1; a dense
+    // pipe's 262,144, before k_density_wc, 23 and 33).
     Launch next = L;
-    if (tasks.list && L.n <= 2048 * device_sm_count()) next.smem_share = 100;
+    if (tasks.tc_next && L.n <= 2048 * device_sm_count()) next.smem_share = 100;
     return launch_chained(pos64 ? k_rank_gather<true> : k_rank_gather<false>, (L.n + b - 1) / b, b,
                           next, L.n, cell, pid, tmp_pid, vstart, vcount, pos, vel, pos64, pos_out,
                           vel_out, pid_out, pos64_out, tasks, L.big_voxel, slot, L.pbegin,

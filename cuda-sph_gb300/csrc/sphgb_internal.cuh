@@ -724,6 +724,7 @@ struct TaskLists {
     int32_t* tc_count = nullptr;
     int tc_max = 0;      // one list
     int pair_max = 0;    // 0: none
+    bool tc_next = false;    // k_density_tc is the kernel after the rank-gather
 };
 // tmp_pid must be 16-byte aligned with 4 entries of room past n (the rank
 // count reads it in aligned quads).
