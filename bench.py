@@ -53,14 +53,10 @@ for _p in (os.path.join(ROOT, "cuda-sph_gb300"), ROOT):
 STAGE_BYTES_PER_PARTICLE = {"hash": 20, "scan": 0, "scatter": 8, "rank_gather": 48,
                             "density": 16, "force_integrate": 100, "step_counter": 0}
 STAGE_BYTES_PER_VOXEL = {"hash": 4, "scan": 8}
-# kernels per step: hash, scan (2; 3 for voxel tables over 8192 x 4096 entries),
-# scatter, big-voxel sort, rank-gather, density, force+integrate, step counter
-def kernels_per_step(n_voxels):
-    """Our kernels per fused step of a box context: hash, tile reduce, tile
-    scan (plus the one-block scan of the tile sums above 8192 tiles), scatter,
-    big-voxel sort, rank-gather, density, the force pass's two launches (the
-    list path, then the deferred particles) and the step counter."""
-    return 10 if (n_voxels + 4095) // 4096 <= 8192 else 11
+# Our kernels per fused step of one kind of scene: hash, scan, scatter, big-voxel
+# sort, rank-gather, density, and the force pass's two launches (the list path,
+# then the deferred particles; pipe scenes: one, and the step counter).
+KERNELS_PER_STEP = 8
 
 
 _T0 = time.perf_counter()
@@ -219,14 +215,20 @@ def measured_peak_hbm():
         return 6800.0, "fallback"
 
 
+def profile_path(stage, workload):
+    """The committed ncu summary of a stage's kernel on a workload (dense scenes
+    run k_density_wc)."""
+    names = {"force_integrate": "k_integrate", "rank_gather": "k_rank_gather",
+             "density": "k_density_wc" if workload == "config1" else "k_density_tc"}
+    return os.path.join("profiles", f"{names.get(stage, stage)}_{workload}.md")
+
+
 def committed_inst_per_particle(stage, workload="config2"):
     """Warp instructions per particle of a stage's kernel from the committed ncu
     summary of this workload (its '... N warp instructions per particle.'
     line), or None when there is none."""
     import re
-    names = {"force_integrate": "k_integrate", "density": "k_density_wc",
-             "rank_gather": "k_rank_gather"}
-    p = os.path.join(ROOT, "profiles", f"{names.get(stage, stage)}_{workload}.md")
+    p = os.path.join(ROOT, profile_path(stage, workload))
     try:
         m = re.search(r"(\d+) warp instructions per particle", open(p).read())
         return int(m.group(1)) if m else None
@@ -238,9 +240,7 @@ def committed_traffic(stage, workload="config2"):
     """DRAM bytes per launch of a stage's kernel from the committed ncu summary
     of this workload (profiles/<kernel>_<workload>.md, line
     'traffic_bytes_per_launch: X'), or None when there is none."""
-    names = {"force_integrate": "k_integrate", "density": "k_density_wc",
-             "rank_gather": "k_rank_gather"}
-    p = os.path.join(ROOT, "profiles", f"{names.get(stage, stage)}_{workload}.md")
+    p = os.path.join(ROOT, profile_path(stage, workload))
     try:
         for line in open(p):
             if line.startswith("traffic_bytes_per_launch:"):
@@ -254,9 +254,7 @@ def profile_source(stage, workload="config2"):
     """Where the committed per-kernel figures (DRAM traffic, warp
     instructions) come from: the ncu summary file and the case it captured,
     read from its 'case:' line.  These figures are not measured in this run."""
-    names = {"force_integrate": "k_integrate", "density": "k_density_wc",
-             "rank_gather": "k_rank_gather"}
-    rel = os.path.join("profiles", f"{names.get(stage, stage)}_{workload}.md")
+    rel = profile_path(stage, workload)
     case = None
     try:
         for line in open(os.path.join(ROOT, rel)):
@@ -494,7 +492,7 @@ def run_gb300(args):
            "autotune": {"chosen": {"density": {0: "warp", 1: "thread"}[best.density_variant],
                                    "sort_block": best.sort_block, "big_voxel": best.big_voxel},
                         "ms_per_step": summary(tried)},
-           "clocks": clocks, "gpu_launches": kernels_per_step(batch.n_voxels) * args.steps}
+           "clocks": clocks, "gpu_launches": KERNELS_PER_STEP * args.steps}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         out["cpu_baseline"], want = cpu_baseline(spec, state, max(args.cpu_steps, 1),
                                                  step_index=e2e_step)

@@ -37,10 +37,10 @@ namespace {
 // distance with the walk's FP32 arithmetic, density term, Kahan sum.  The sum
 // is that of density_one, so both kernels give the same bits.
 //
-// What bounds it: instruction issue (69 % of the issue slots with 24 warps per
-// SM) beside shared memory (67 % of its wavefronts).  A 4,194,304-particle box
+// What bounds it: instruction issue (70 % of the issue slots with 24 warps per
+// SM) beside the L1 / shared-memory pipe (76 %).  A 4,194,304-particle box
 // at 11 particles per voxel: 1.171 ms with the ballots and per-home ranking of
-// k_density_wc, 0.948 ms here, 2765 against 2000 warp instructions per task of
+// k_density_wc, 0.940 ms here, 2765 against 2000 warp instructions per task of
 // 10 homes (400 to set up, 100 per group of candidates for all homes, 760 in
 // phase 2).  262,144 particles: 88 -> 71 us.  Measured and not kept: 32 warps per
 // SM at 64 registers (1.09 ms: spills, 20 % more instructions), 16-bit list

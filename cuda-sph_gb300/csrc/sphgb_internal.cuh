@@ -716,7 +716,7 @@ constexpr int kTaskRun = 16;
 // indices differ in bit 4.  k_density_tc pays most of a task's cost per task,
 // not per particle, and two voxels' walks share half their voxels: 48 boxes of
 // 8 particles per voxel, 699,220 in all, 235 -> 146 us of density; a box of
-// 4,194,304 at 11 per voxel, where few pairs fit, 993 -> 948.
+// 4,194,304 at 11 per voxel, where few pairs fit, 993 -> 940.
 struct TaskLists {
     int2* list = nullptr;
     int32_t* count = nullptr;
