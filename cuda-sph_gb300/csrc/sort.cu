@@ -40,27 +40,6 @@ __device__ __forceinline__ int warp_incl_scan(int v) {
     return v;
 }
 
-// exclusive scan of one int per thread across the block; `total` receives the
-// block total.  Safe to call repeatedly if the caller synchronises between calls.
-__device__ __forceinline__ int block_excl_scan(int v, int& total) {
-    constexpr int kWarps = kScanThreads / 32;
-    __shared__ int warp_off[kWarps];
-    __shared__ int block_total;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int incl = warp_incl_scan(v);
-    if (lane == 31) warp_off[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        const int w = lane < kWarps ? warp_off[lane] : 0;
-        const int wi = warp_incl_scan(w);
-        if (lane < kWarps) warp_off[lane] = wi - w;
-        if (lane == kWarps - 1) block_total = wi;
-    }
-    __syncthreads();
-    total = block_total;
-    return incl - v + warp_off[wid];
-}
-
 __global__ void __launch_bounds__(512)
 k_hash_count(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin, int n_scenes,
              int i0, int i1, const float4* __restrict__ pos, int32_t* __restrict__ cell,
@@ -151,27 +130,46 @@ __device__ __forceinline__ int look_back(const int32_t* __restrict__ vcount, int
 __global__ void __launch_bounds__(kScanThreads)
 k_scan(const int32_t* __restrict__ vcount, int v_total, unsigned long long* status,
        int32_t* __restrict__ vstart, int4* __restrict__ next_counts, int next_quads) {
-    __shared__ int s_before;
+    __shared__ int s_before, s_warp[kScanThreads / 32];
     const int tile = grid_wait((int)blockIdx.x);
-    const int base = tile * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // A warp's part of the tile in rows of 128, four entries per lane in each: whole
+    // lines per access, where a lane's 16 entries in a row wrote half sectors, and
+    // one barrier instead of two (699,220 particles in 48 boxes, 2.5 M entries:
+    // stage 15.1 -> 13.3 us; step of 8,192 particles 26.0 -> 25.2).
+    const int base = tile * kScanTile + wid * (32 * kScanItems) + 4 * lane;
+    constexpr int kRows = kScanItems / 4;
+    int4 v[kRows];
     const bool full = (tile + 1) * kScanTile <= v_total;
-    if (full) {
-        const int4* v4 = reinterpret_cast<const int4*>(vcount + base);
 #pragma unroll
-        for (int i = 0; i < kScanItems / 4; ++i) {
-            int4 q = __ldg(v4 + i);
-            v[4 * i] = q.x; v[4 * i + 1] = q.y; v[4 * i + 2] = q.z; v[4 * i + 3] = q.w;
+    for (int i = 0; i < kRows; ++i) {
+        const int k = base + 128 * i;
+        if (full) {
+            v[i] = __ldg(reinterpret_cast<const int4*>(vcount + k));
+        } else {
+            v[i].x = k < v_total ? __ldg(vcount + k) : 0;
+            v[i].y = k + 1 < v_total ? __ldg(vcount + k + 1) : 0;
+            v[i].z = k + 2 < v_total ? __ldg(vcount + k + 2) : 0;
+            v[i].w = k + 3 < v_total ? __ldg(vcount + k + 3) : 0;
         }
-    } else {
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) v[i] = base + i < v_total ? __ldg(vcount + base + i) : 0;
     }
-    int tsum = 0;
+    int excl[kRows], in_warp = 0;
 #pragma unroll
-    for (int i = 0; i < kScanItems; ++i) tsum += v[i];
-    int total = 0;
-    const int excl = block_excl_scan(tsum, total);
+    for (int i = 0; i < kRows; ++i) {
+        const int sum = v[i].x + v[i].y + v[i].z + v[i].w;
+        const int incl = warp_incl_scan(sum);
+        excl[i] = in_warp + incl - sum;
+        in_warp += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_warp[wid] = in_warp;
+    __syncthreads();
+    int before_warp = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+        const int t = s_warp[w];
+        before_warp += w < wid ? t : 0;
+        total += t;
+    }
     if (threadIdx.x < 32) {
         volatile unsigned long long* mine = status + tile;
         if (threadIdx.x == 0) *mine = (tile ? kScanSum : kScanPrefix) | (unsigned)total;
@@ -186,18 +184,23 @@ k_scan(const int32_t* __restrict__ vcount, int v_total, unsigned long long* stat
         }
     }
     __syncthreads();
-    int run = excl + s_before;
-    int out[kScanItems];
+    const int off = before_warp + s_before;
 #pragma unroll
-    for (int i = 0; i < kScanItems; ++i) { out[i] = run; run += v[i]; }
-    if (full) {
-        int4* o4 = reinterpret_cast<int4*>(vstart + base);
-#pragma unroll
-        for (int i = 0; i < kScanItems / 4; ++i)
-            o4[i] = make_int4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) if (base + i < v_total) vstart[base + i] = out[i];
+    for (int i = 0; i < kRows; ++i) {
+        const int k = base + 128 * i;
+        int4 o;
+        o.x = off + excl[i];
+        o.y = o.x + v[i].x;
+        o.z = o.y + v[i].y;
+        o.w = o.z + v[i].z;
+        if (full) {
+            *reinterpret_cast<int4*>(vstart + k) = o;
+        } else {
+            if (k < v_total) vstart[k] = o.x;
+            if (k + 1 < v_total) vstart[k + 1] = o.y;
+            if (k + 2 < v_total) vstart[k + 2] = o.z;
+            if (k + 3 < v_total) vstart[k + 3] = o.w;
+        }
     }
     // the next step's counters, status words and counts
     for (int k = blockIdx.x * kScanThreads + threadIdx.x; k < next_quads; k += gridDim.x * kScanThreads)
