@@ -266,6 +266,9 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
            int32_t* __restrict__ tmp_pid) {
     __shared__ alignas(16) int32_t sm[kSmemSort];
     const int nb = *grid_wait(big_count);
+    // most steps: nothing to do (51,911 particles: step 47.4 us through the barrier
+    // below, 45.6 so)
+    if (nb == 0) return;
     const int quarter = threadIdx.x / kQuarter, t = threadIdx.x % kQuarter;
     int32_t* sq = sm + quarter * kRankSort;
     for (int b = blockIdx.x * 4 + quarter; b < nb; b += gridDim.x * 4) {
