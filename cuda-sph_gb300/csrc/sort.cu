@@ -247,8 +247,10 @@ __device__ __forceinline__ void bitonic_pass(int32_t* a, int c, int n2, int k, i
 }
 
 // Segments up to kRankSort ids take a quarter of a block each and no sorting
-// network: every id counts the smaller ones (the ids are distinct), from shared
-// memory four at a time, all threads reading the same quad.  A network of 1024
+// network: every id counts the smaller ones, from shared memory four at a time,
+// all threads reading the same quad.  Equal ids (a caller's mistake) count by
+// place, so the segment is sorted whatever the ids are: the rank-gather's binary
+// search ends inside the voxel only in a sorted one.  A network of 1024
 // threads per voxel spends its time in barriers (36 for 133 ids): the 4,000
 // voxels of ~133 particles of the 262,144-particle pipe took 86 us, 13 us this
 // way.  Beyond 512 ids the counting grows past the network (the pipe's later
@@ -280,8 +282,20 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
         quarter_sync(quarter);
         for (int i = t; i < c; i += kQuarter) {
             const int32_t p = sq[i];
+            // the warp's own 32 ids lie between those that come before all of
+            // its ids and those that come after: equal ids keep their order
+            const int own = i & ~31, after = min(own + 32, c4);
             int r = 0;
-            for (int k = 0; k < c4; k += 4) {
+            for (int k = 0; k < own; k += 4) {
+                const int4 q = *reinterpret_cast<const int4*>(sq + k);
+                r += (q.x <= p) + (q.y <= p) + (q.z <= p) + (q.w <= p);
+            }
+            for (int k = own; k < after; k += 4) {
+                const int4 q = *reinterpret_cast<const int4*>(sq + k);
+                r += (q.x < p || (q.x == p && k < i)) + (q.y < p || (q.y == p && k + 1 < i)) +
+                     (q.z < p || (q.z == p && k + 2 < i)) + (q.w < p || (q.w == p && k + 3 < i));
+            }
+            for (int k = after; k < c4; k += 4) {
                 const int4 q = *reinterpret_cast<const int4*>(sq + k);
                 r += (q.x < p) + (q.y < p) + (q.z < p) + (q.w < p);
             }
