@@ -1845,9 +1845,12 @@ constexpr size_t kDirectPinned = 131072;
 constexpr size_t kDirectPaged = 40000;
 
 // the address under which kernels reach a host buffer, or null; paged is set
-// when it is ordinary (not page-locked) memory
+// when it is ordinary (not page-locked) memory.  Copies take a buffer at any
+// byte address (an array that views a file behind a header of 4 bytes), kernels
+// only at whole doubles.
 template <class T>
 T* device_view(T* h, bool& paged) {
+    if (reinterpret_cast<uintptr_t>(h) % sizeof(T) != 0) return nullptr;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, h) != cudaSuccess) {
         cudaGetLastError();
