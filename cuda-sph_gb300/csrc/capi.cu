@@ -191,17 +191,17 @@ struct SphgbCtx {
     double* stage = nullptr;
     // neighbour lists of the stage entry points (stage_lists), allocated on their
     // first call and given back with the scenes they were sized for; apart from
-    // the step's own, which sphgb_ctx_step_neighbours reads after stage calls.
-    // lists_ev: the stream of the last call is done with them.
+    // the step's own, which sphgb_ctx_step_neighbours reads after stage calls
     struct {
         int2* tasks = nullptr;
         int32_t* words = nullptr;       // 64 counters (tasks, taken, bad), rows, counts
         int32_t* over = nullptr;
         bool failed = false;            // no memory: the stages walk
-        cudaEvent_t ev = nullptr;
-        cudaStream_t last = nullptr;
-        bool used = false;
     } lists;
+    // the stage call before this one is done with what they share (StageScope)
+    cudaEvent_t stage_ev = nullptr;
+    cudaStream_t stage_last = nullptr;
+    bool stage_used = false;
     // conservation
     int n_chunks = 0;
     ConsChunk* d_chunks = nullptr;
@@ -331,7 +331,6 @@ void free_lists(SphgbCtx* c) {
     if (c->lists.tasks) cudaFree(c->lists.tasks);
     if (c->lists.words) cudaFree(c->lists.words);
     if (c->lists.over) cudaFree(c->lists.over);
-    if (c->lists.ev) cudaEventDestroy(c->lists.ev);
     c->lists = {};
 }
 
@@ -350,6 +349,7 @@ void free_ctx(SphgbCtx* c) {
     if (c->host_stream) cudaStreamDestroy(c->host_stream);
     if (c->host_stream2) cudaStreamDestroy(c->host_stream2);
     if (c->host_stream4) cudaStreamDestroy(c->host_stream4);
+    if (c->stage_ev) cudaEventDestroy(c->stage_ev);
     for (cudaEvent_t e : c->pipe_ev)
         if (e) cudaEventDestroy(e);
     if (c->tasks_b) cudaFree(c->tasks_b);
@@ -867,24 +867,54 @@ int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int rang
     return SPHGB_OK;
 }
 
+// The stage calls of a context share its force records and neighbour lists,
+// whatever streams they are on: each waits for the one before it, before its
+// first launch.  Not under stream capture, where an event of this kind has no
+// place; such a call's lists are empty (stage_lists).
+struct StageScope {
+    SphgbCtx* c;
+    cudaStream_t st;
+    bool captured = false, on = false;
+    StageScope(SphgbCtx* c_, cudaStream_t st_) : c(c_), st(st_) {}
+    StageScope(const StageScope&) = delete;
+    int begin() {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+            cudaGetLastError();       // the legacy stream beside a capture elsewhere
+            captured = true;
+        } else {
+            captured = cap != cudaStreamCaptureStatusNone;
+        }
+        if (captured) return SPHGB_OK;
+        if (!c->stage_ev)
+            SPHGB_CUDA(cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming));
+        if (c->stage_used && c->stage_last != st)
+            SPHGB_CUDA(cudaStreamWaitEvent(st, c->stage_ev, 0));
+        c->stage_used = true;
+        c->stage_last = st;
+        on = true;
+        return SPHGB_OK;
+    }
+    int end() {
+        if (on) SPHGB_CUDA(cudaEventRecord(c->stage_ev, st));
+        return SPHGB_OK;
+    }
+};
+
 // Neighbour lists of the sorted state and voxel table of a stage call, by the
 // step's density passes, which also write the densities when rho is given.
 // Returns the lists, or empty ones where the stage has to walk as it did before
 // there were lists: under stream capture (the first call allocates, and calls
 // are ordered by an event) and without memory.  Lists of a table that is not
 // the state's are vetoed on the device.
-int stage_lists(SphgbCtx* c, const Launch& L, const float4* pos, const int32_t* vstart,
-                const int32_t* vcount, float* rho, NbrList& out, int32_t*& bad) {
+int stage_lists(SphgbCtx* c, const StageScope& scope, const Launch& L, const float4* pos,
+                const int32_t* vstart, const int32_t* vcount, float* rho, NbrList& out,
+                int32_t*& bad) {
     out = NbrList{};
     bad = nullptr;
     const size_t N = (size_t)c->n;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(L.stream, &cap) != cudaSuccess) {
-        cudaGetLastError();       // the legacy stream beside a capture elsewhere
-        return SPHGB_OK;
-    }
     auto& l = c->lists;
-    if (cap != cudaStreamCaptureStatusNone || l.failed || N == 0) return SPHGB_OK;
+    if (scope.captured || l.failed || N == 0) return SPHGB_OK;
     const size_t head = kCountersPad;
     if (!l.words) {
         // allowed beside a capture of another stream or thread
@@ -893,10 +923,6 @@ int stage_lists(SphgbCtx* c, const Launch& L, const float4* pos, const int32_t* 
         int rc = dalloc(&l.tasks, N);
         if (!rc) rc = dalloc(&l.words, head + (kListCap + 1) * N + 8);
         if (!rc && c->uncapped) rc = dalloc(&l.over, 8 * (size_t)std::min(N * kOverPerParticle, kOverMax));
-        if (!rc && cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            rc = SPHGB_ERR_CUDA;
-        }
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (rc) {
             free_lists(c);
@@ -905,9 +931,6 @@ int stage_lists(SphgbCtx* c, const Launch& L, const float4* pos, const int32_t* 
             return SPHGB_OK;
         }
     }
-    if (l.used && l.last != L.stream) SPHGB_CUDA(cudaStreamWaitEvent(L.stream, l.ev, 0));
-    l.used = true;
-    l.last = L.stream;
     SPHGB_CUDA(cudaMemsetAsync(l.words, 0, sizeof(int32_t) * head, L.stream));
     bad = l.words + 2;
     out.idx = l.words + head;
@@ -926,11 +949,6 @@ int stage_lists(SphgbCtx* c, const Launch& L, const float4* pos, const int32_t* 
     else
         SPHGB_CUDA(launch_density_tc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks, 1,
                                      l.words, l.words + 1, c->uncapped));
-    return SPHGB_OK;
-}
-// the stage is done with the lists
-int stage_lists_end(SphgbCtx* c, const NbrList& l, cudaStream_t st) {
-    if (l.count) SPHGB_CUDA(cudaEventRecord(c->lists.ev, st));
     return SPHGB_OK;
 }
 
@@ -2272,15 +2290,18 @@ int sphgb_density(SphgbCtx* ctx, const float* d_pos_sorted, const int32_t* d_vox
     if (ctx->n > 0 && (!d_pos_sorted || !d_rho_out)) return fail(SPHGB_ERR_INVALID, "null buffer");
     cudaStream_t st = as_stream(stream);
     const Launch L = ctx->launch(st, true);
+    StageScope scope(ctx, st);
+    int rc = scope.begin();
+    if (rc) return rc;
     const float4* pos = reinterpret_cast<const float4*>(d_pos_sorted);
     NbrList nbr;
     int32_t* bad;
-    int rc = stage_lists(ctx, L, pos, d_voxel_start, d_voxel_count, d_rho_out, nbr, bad);
+    rc = stage_lists(ctx, scope, L, pos, d_voxel_start, d_voxel_count, d_rho_out, nbr, bad);
     if (rc) return rc;
     // without lists, or when they were vetoed: one thread walks per particle
     SPHGB_CUDA(launch_density(L, pos, nullptr, d_voxel_start, d_voxel_count, d_rho_out, nullptr,
                               NbrList{}, bad));
-    return stage_lists_end(ctx, nbr, st);
+    return scope.end();
 }
 
 int sphgb_forces(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel_sorted,
@@ -2293,19 +2314,22 @@ int sphgb_forces(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel_so
         return fail(SPHGB_ERR_INVALID, "null buffer");
     cudaStream_t st = as_stream(stream);
     const Launch L = ctx->launch(st, true);
+    StageScope scope(ctx, st);
+    int rc = scope.begin();
+    if (rc) return rc;
     SPHGB_CUDA(launch_force_inputs(L, reinterpret_cast<const float4*>(d_pos_sorted),
                                    reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted,
                                    ctx->fin));
     NbrList nbr;
     int32_t* bad;
-    int rc = stage_lists(ctx, L, reinterpret_cast<const float4*>(d_pos_sorted), d_voxel_start,
-                         d_voxel_count, nullptr, nbr, bad);
+    rc = stage_lists(ctx, scope, L, reinterpret_cast<const float4*>(d_pos_sorted), d_voxel_start,
+                     d_voxel_count, nullptr, nbr, bad);
     if (rc) return rc;
     SPHGB_CUDA(launch_forces(L, reinterpret_cast<const float4*>(d_pos_sorted),
                              reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted, ctx->fin,
                              d_voxel_start, d_voxel_count, reinterpret_cast<float4*>(d_pressure_out),
                              reinterpret_cast<float4*>(d_viscosity_out), nbr));
-    return stage_lists_end(ctx, nbr, st);
+    return scope.end();
 }
 
 int sphgb_integrate(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel_sorted,
@@ -2322,13 +2346,16 @@ int sphgb_integrate(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel
         return fail(SPHGB_ERR_INVALID, "pipe scenes need the FP64 position buffers");
     cudaStream_t st = as_stream(stream);
     const Launch L = ctx->launch(st, true);
+    StageScope scope(ctx, st);
+    int rc = scope.begin();
+    if (rc) return rc;
     SPHGB_CUDA(launch_force_inputs(L, reinterpret_cast<const float4*>(d_pos_sorted),
                                    reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted,
                                    ctx->fin));
     NbrList nbr;
     int32_t* bad;
-    int rc = stage_lists(ctx, L, reinterpret_cast<const float4*>(d_pos_sorted), d_voxel_start,
-                         d_voxel_count, nullptr, nbr, bad);
+    rc = stage_lists(ctx, scope, L, reinterpret_cast<const float4*>(d_pos_sorted), d_voxel_start,
+                     d_voxel_count, nullptr, nbr, bad);
     if (rc) return rc;
     SPHGB_CUDA(launch_integrate(L, reinterpret_cast<const float4*>(d_pos_sorted),
                                 reinterpret_cast<const float4*>(d_vel_sorted), d_rho_sorted,
@@ -2337,7 +2364,7 @@ int sphgb_integrate(SphgbCtx* ctx, const float* d_pos_sorted, const float* d_vel
                                 reinterpret_cast<float4*>(d_pos_out),
                                 reinterpret_cast<float4*>(d_vel_out), d_pid_out, d_pos64_out,
                                 reinterpret_cast<float4*>(d_force_out)));
-    return stage_lists_end(ctx, nbr, st);
+    return scope.end();
 }
 
 int sphgb_pipe_find_segment(const double* d_pos, int n, const double* d_pipe, int pipe_rows,
