@@ -200,7 +200,7 @@ struct SphgbCtx {
     } lists;
     // the stage call before this one is done with what they share (StageScope)
     cudaEvent_t stage_ev = nullptr;
-    cudaStream_t stage_last = nullptr;
+    unsigned long long stage_last = 0;      // its stream's id
     bool stage_used = false;
     // conservation
     int n_chunks = 0;
@@ -869,14 +869,20 @@ int enqueue_forces(SphgbCtx* c, const Launch& L, const PidRange* range, int rang
 
 // The stage calls of a context share its force records and neighbour lists,
 // whatever streams they are on: each waits for the one before it, before its
-// first launch.  Not under stream capture, where an event of this kind has no
-// place; such a call's lists are empty (stage_lists).
+// first launch.  Streams are told apart by their ids: a handle may be that of a
+// stream that is gone, with the call on it still running.  A call that fails
+// half way is waited for like any other (what it enqueued runs).  Not under
+// stream capture, where an event of this kind has no place; such a call's lists
+// are empty (stage_lists).
 struct StageScope {
     SphgbCtx* c;
     cudaStream_t st;
     bool captured = false, on = false;
     StageScope(SphgbCtx* c_, cudaStream_t st_) : c(c_), st(st_) {}
     StageScope(const StageScope&) = delete;
+    ~StageScope() {
+        if (on && cudaEventRecord(c->stage_ev, st) != cudaSuccess) cudaGetLastError();
+    }
     int begin() {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
@@ -888,15 +894,19 @@ struct StageScope {
         if (captured) return SPHGB_OK;
         if (!c->stage_ev)
             SPHGB_CUDA(cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming));
-        if (c->stage_used && c->stage_last != st)
+        unsigned long long id = 0;
+        SPHGB_CUDA(cudaStreamGetId(st, &id));
+        if (c->stage_used && c->stage_last != id)
             SPHGB_CUDA(cudaStreamWaitEvent(st, c->stage_ev, 0));
         c->stage_used = true;
-        c->stage_last = st;
+        c->stage_last = id;
         on = true;
         return SPHGB_OK;
     }
     int end() {
-        if (on) SPHGB_CUDA(cudaEventRecord(c->stage_ev, st));
+        if (!on) return SPHGB_OK;
+        on = false;
+        SPHGB_CUDA(cudaEventRecord(c->stage_ev, st));
         return SPHGB_OK;
     }
 };

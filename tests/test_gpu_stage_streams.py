@@ -59,3 +59,28 @@ def test_streams_that_nothing_else_orders():
                 got[k] += K.integrate(b, *integ)
         _compare(got, cases)
     b.close()
+
+
+def test_streams_that_come_and_go():
+    """Every call on a stream of its own, destroyed with the call on it: the next
+    stream may have the same handle."""
+    torch = torch_cuda()
+    import ctypes
+    from sphgb import kernels as K
+    from sphgb.device import SceneBatch
+    from test_gpu_density_paths import _spec
+    n = 60_000
+    b = SceneBatch([_spec(n, (1.0, 1.0, 1.0), 0.05, 32)])
+    cases = _inputs(b, n, range(3))
+    rt = torch.cuda.cudart()
+    got = [[] for _ in cases]
+    for call in (K.pressure_viscosity, K.integrate):
+        for k, (pv, integ, _) in enumerate(cases):
+            handle = ctypes.c_void_p()
+            assert int(rt.cudaStreamCreate(ctypes.addressof(handle))) == 0
+            # the outputs belong to the test's own stream, whose memory outlives the call
+            got[k] += call(b, *(pv if call is K.pressure_viscosity else integ),
+                           stream=torch.cuda.ExternalStream(handle.value))
+            assert int(rt.cudaStreamDestroy(handle.value)) == 0
+    _compare(got, cases)
+    b.close()
