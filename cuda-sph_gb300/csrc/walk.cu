@@ -1168,8 +1168,13 @@ cudaError_t launch_force_pass(const Launch& L, int m, const float4* pos, const f
                 : launch(k_integrate<false, kIdx, kForceLean>, grid, rare, nullptr);
         if (e != cudaSuccess) return e;
         Lf.chained = L.chained;
+        // four blocks per SM, all resident: the deferred particles may be most of a
+        // scene (no cap, lists longer than their pool), and their walks wait for
+        // loads.  100,000 particles with 167 neighbours: force pass 1538 us with one
+        // block per SM, 725 with four; steps without a deferred particle the same.
         return launch(k_integrate<false, kIdx, kForceRare>,
-                      std::min(blocks_for(std::max(m, L.n_scenes)), device_sm_count()), rare, advance);
+                      std::min(blocks_for(std::max(m, L.n_scenes)), 4 * device_sm_count()), rare,
+                      advance);
     }
     return launch(k_integrate<false, kIdx, kForceAll>, grid, RareList{}, nullptr);
 }
