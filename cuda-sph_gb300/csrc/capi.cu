@@ -946,7 +946,7 @@ int stage_lists(SphgbCtx* c, const StageScope& scope, const Launch& L, const flo
     out.idx = l.words + head;
     out.count = out.idx + kListCap * N;
     out.veto = bad;
-    if (c->uncapped) {
+    if (c->uncapped && !rho) {      // the density call reads no list
         out.over = l.over;
         out.over_used = reinterpret_cast<unsigned long long*>(l.words + kOverCounter);
         out.over_units = std::min(N * kOverPerParticle, kOverMax);

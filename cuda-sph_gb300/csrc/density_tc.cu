@@ -356,14 +356,15 @@ __device__ __forceinline__ uint32_t drop_first(uint32_t w, int d) {
 
 // Phase 2 for one lane: visits the next n accepted candidates of its home,
 // adds their density terms and stores their slots from shared-memory address
-// `row` on (kBound: below row_end only, and into `over` from `row` on when
-// given), passing over the one at address `self`; returns where the row ends.
+// `row` on (kBound: below row_end only, and below over_end from `over` on),
+// passing over the one at address `self`; returns where the row ends.
 // The words hold at least n more bits: n counts bits of theirs.  A lane that
 // meets an empty word lets a turn pass.
 template <bool kBound>
 __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uint32_t row_end,
                                            uint32_t self, const float4& pi, float inv_h2,
-                                           Kahan& acc, int32_t* over = nullptr) {
+                                           Kahan& acc, int32_t* over = nullptr,
+                                           uint32_t over_end = 0u) {
     while (n > 0) {
         C.advance_if_empty();
         // place of the first bit; -1 in an empty word, which is never the
@@ -387,7 +388,10 @@ __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uin
             acc = a;
             if (!kBound || row < row_end)
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(row), "f"(pj.w) : "memory");
-            if (kBound && over) *over++ = __float_as_int(pj.w);
+            if (kBound) {
+                if (row < over_end) *over = __float_as_int(pj.w);
+                ++over;
+            }
             row += 4;
         }
     }
@@ -583,28 +587,62 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         int others = 0;    // of those, not the particle itself
         Kahan acc;         // lane i: entries of home i below kSumSplit, lane 16 + i: the rest
         Kahan first;       // uncapped: the first part; acc of lane i then sums every entry
-        long long unit = -1;     // uncapped: the home's place in the pool
+        long long unit = 0;      // uncapped: the home's place in the pool, and its length
+        int room = 0;
+        // Uncapped: the lists that will not fit their rows get room in the pool, as
+        // long as the accepted candidates and those of the walk that are still
+        // to come.  More of those than a batch, and the walk is decided twice,
+        // once to count (counting) and again, chunk by chunk, to list; not when
+        // the pool is full.  Room for the rest of any walk, uncounted, left most
+        // particles of scenes of 12 and more per voxel without a list (100,000
+        // particles, step: 13 per voxel 426 -> 186 us, 20: 632 -> 271).
+        bool counting = false, reserve = kUncapped && uncapped && nbr.over;
+        if (kUncapped && reserve && M > kTcChunk + kTcBatch) {
+            int left = 0;
+            if (lane == 0)
+                left = *(volatile unsigned long long*)nbr.over_used < nbr.over_units;
+            counting = reserve = __shfl_sync(full, left, 0);
+        }
         for (int c0 = 0; c0 < M; c0 += kTcChunk) {
             const int c1 = min(M, c0 + kTcChunk);
             int T, gh, Th;
             const int G = tc_decide(S, T, gh, Th, cnt, c_t, cap, c0, c1, W, cull, A, Cq, ballots, F, pi,
                                     pos, n, sc);
-            if (uncapped && c0 == 0 && nbr.over) {
-                // room for the lists that will not fit their rows: of known
-                // length when this chunk is the walk, else as long as the walk
-                const int most = c1 == M ? T : M;
-                const int need = home && most > kListCap ? (most + 7) >> 3 : 0;
-                int incl = need;
+            if (kUncapped && reserve) {
+                const int seen = min(cnt + T, cap);
+                const bool all = !counting || c1 == M || !__any_sync(full, home && seen < cap);
+                if (all) {
+                    const int most = counting ? seen : min(cnt + T + M - c1, cap);
+                    const int need = home && most > kListCap ? (most + 7) >> 3 : 0;
+                    int incl = need;
 #pragma unroll
-                for (int o = 1; o < kTaskRun; o <<= 1) {
-                    const int v = __shfl_up_sync(full, incl, o);
-                    if (lane >= o) incl += v;
+                    for (int o = 1; o < kTaskRun; o <<= 1) {
+                        const int v = __shfl_up_sync(full, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    const int total = __shfl_sync(full, incl, kTaskRun - 1);
+                    unsigned long long u = 0;
+                    if (lane == 0 && total) u = atomicAdd(nbr.over_used, (unsigned long long)total);
+                    u = __shfl_sync(full, u, 0);
+                    if (need && u + total <= nbr.over_units) {
+                        unit = (long long)u + incl - need;
+                        room = 8 * need;
+                    }
+                    reserve = false;
                 }
-                const int total = __shfl_sync(full, incl, kTaskRun - 1);
-                unsigned long long u = 0;
-                if (lane == 0 && total) u = atomicAdd(nbr.over_used, (unsigned long long)total);
-                u = __shfl_sync(full, u, 0);
-                if (u + total <= nbr.over_units) unit = need ? (long long)u + incl - need : -1;
+                if (counting) {
+                    cnt = seen;
+                    if (!all) continue;
+                    counting = false;
+                    cnt = 0;
+                    __syncwarp();       // every lane is done with the marks
+                    if (lane < kTcWords) S.seg[lane] = 0u;
+                    __syncwarp();
+                    W.mark(S, 0);
+                    __syncwarp();
+                    c0 = -kTcChunk;
+                    continue;
+                }
             }
             const int n_all = ih < c_t ? max(min(T, cap - cnt), 0) : 0;   // entries used here
             int n_lo = min(n_all, max(kSumSplit - cnt, 0)), n_hi = n_all - n_lo;
@@ -629,11 +667,14 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             } else {
                 // the lower lane goes over every entry and lists them
                 const uint32_t row_end = upper ? row0 : row0 + 4 * kListCap;
-                int32_t* over = unit >= 0 ? nbr.over + 8 * unit + others : nullptr;    // lower lanes
-                end = tc_sum<true>(C, upper ? n_hi : n_lo, row, row_end, self, pi, inv_h2, acc, over);
+                int32_t* over = nbr.over + 8 * unit + others;    // lower lanes
+                const uint32_t over_end = row0 + 4 * room;
+                end = tc_sum<true>(C, upper ? n_hi : n_lo, row, row_end, self, pi, inv_h2, acc, over,
+                                   over_end);
                 if (cnt < kSumSplit) first = acc;
-                if (over) over += (end - row) >> 2;
-                end = tc_sum<true>(C, upper ? 0 : n_hi, end, row_end, self, pi, inv_h2, acc, over);
+                over += (end - row) >> 2;
+                end = tc_sum<true>(C, upper ? 0 : n_hi, end, row_end, self, pi, inv_h2, acc, over,
+                                   over_end);
             }
             // entries of both lanes (uncapped: the lower lane went over all)
             const int mine = (int)(end - row) >> 2;
@@ -646,7 +687,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         __syncwarp();
         if (lane < kTcWords) S.seg[lane] = 0u;      // for the next task
         if (kUncapped && home && others > kListCap) {
-            S.list[ih][0] = unit >= 0 ? others : 0;
+            S.list[ih][0] = others <= room ? others : 0;
             S.list[ih][1] = (int)unit;
         }
         if (kUncapped) __syncwarp();
