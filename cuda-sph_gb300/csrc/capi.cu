@@ -194,7 +194,7 @@ struct SphgbCtx {
     // the step's own, which sphgb_ctx_step_neighbours reads after stage calls
     struct {
         int2* tasks = nullptr;
-        int32_t* words = nullptr;       // 64 counters (tasks, taken, bad), rows, counts
+        int32_t* words = nullptr;       // 64 counters (see stage_lists), rows, counts
         int32_t* over = nullptr;
         bool failed = false;            // no memory: the stages walk
     } lists;
@@ -946,12 +946,16 @@ int stage_lists(SphgbCtx* c, const StageScope& scope, const Launch& L, const flo
     out.idx = l.words + head;
     out.count = out.idx + kListCap * N;
     out.veto = bad;
+    StageRoom room;
     if (c->uncapped && !rho) {      // the density call reads no list
         out.over = l.over;
         out.over_used = reinterpret_cast<unsigned long long*>(l.words + kOverCounter);
         out.over_units = std::min(N * kOverPerParticle, kOverMax);
+        room.limit = 8 * out.over_units;
+        room.entries = reinterpret_cast<unsigned long long*>(l.words + kOverCounter - 2);
+        room.blocks = l.words + 3;
     }
-    SPHGB_CUDA(launch_stage_tasks(L, pos, vstart, vcount, l.tasks, l.words, bad));
+    SPHGB_CUDA(launch_stage_tasks(L, pos, vstart, vcount, l.tasks, l.words, bad, room));
     // dense scenes: see density_pass
     if (c->density_pass() == SphgbCtx::kPassWc)
         SPHGB_CUDA(launch_density_wc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks,

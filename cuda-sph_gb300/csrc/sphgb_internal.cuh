@@ -744,10 +744,19 @@ cudaError_t launch_density(const Launch& L, const float4* pos, const float4* vel
 // stage entry points), as the rank-gather lists them.  bad is set, and the
 // density passes given nbr.veto = bad do nothing, when the table is not that
 // of the state: some particle's slot outside its voxel's range, or a range that
-// is not one voxel's.
+// is not one voxel's.  room (scenes without a cap): bad is set too when the
+// lists would be longer than `limit` entries together, taking every voxel's
+// surroundings for as full as itself.  Lists that go
+// back to a walk for want of room cost both (97,000 particles of 557 neighbours,
+// sphgb_forces: walks 1414 us, lists for some and walks for the others 2656).
+struct StageRoom {
+    unsigned long long limit = 0;               // 0: not asked
+    unsigned long long* entries = nullptr;      // zero before the launch, as is blocks
+    int32_t* blocks = nullptr;
+};
 cudaError_t launch_stage_tasks(const Launch& L, const float4* pos, const int32_t* vstart,
                                const int32_t* vcount, int2* tasks, int32_t* task_count,
-                               int32_t* bad);
+                               int32_t* bad, StageRoom room = StageRoom{});
 // the step's density pass: one warp per task (<= kTaskRun particles of one voxel);
 // task_next: a zeroed counter from which the warps take the tasks
 // task_offset (optional, device): the tasks start at tasks[*task_offset] (one

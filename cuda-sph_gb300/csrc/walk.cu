@@ -434,26 +434,51 @@ __global__ void __launch_bounds__(kBlock)
 k_stage_tasks(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin, int n_scenes,
               int n, const float4* __restrict__ pos, const int32_t* __restrict__ vstart,
               const int32_t* __restrict__ vcount, int2* __restrict__ tasks,
-              int32_t* __restrict__ task_count, int32_t* __restrict__ bad) {
+              int32_t* __restrict__ task_count, int32_t* __restrict__ bad, StageRoom room) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const SceneDev& sc = scenes[scene_of(s, pbegin, n_scenes)];
-    auto voxel = [&](int slot) {
-        const float4 p = __ldg(pos + slot);
-        if (!finite3(p)) return sc.v_begin + sc.v_count;
-        return sc.v_begin + voxel_index(voxel_coord(p.x, sc.vs[0], sc.dims[0]),
-                                        voxel_coord(p.y, sc.vs[1], sc.dims[1]),
-                                        voxel_coord(p.z, sc.vs[2], sc.dims[2]), sc.tiled, sc.dims[0],
-                                        sc.dims[1], sc.nt0, sc.nt1);
-    };
-    const int vid = voxel(s);
-    const int st = __ldg(vstart + vid), c = __ldg(vcount + vid);
-    // the slot in its voxel's range, the range inside the scene; the slot before
-    // it in the same voxel; and the range's last slot, seen from its first
-    bool ok = s >= st && s - st < c && st >= sc.p_begin && c <= sc.p_begin + sc.p_count - st;
-    if (ok) ok = s > st ? voxel(s - 1) == vid : voxel(st + c - 1) == vid;
-    if (!ok) atomicOr(bad, 1);
-    else if ((s - st) % kTaskRun == 0) tasks[atomicAdd(task_count, 1)] = make_int2(vid, s);
+    unsigned entries = 0;
+    if (s < n) {
+        const SceneDev& sc = scenes[scene_of(s, pbegin, n_scenes)];
+        auto voxel = [&](int slot) {
+            const float4 p = __ldg(pos + slot);
+            if (!finite3(p)) return sc.v_begin + sc.v_count;
+            return sc.v_begin + voxel_index(voxel_coord(p.x, sc.vs[0], sc.dims[0]),
+                                            voxel_coord(p.y, sc.vs[1], sc.dims[1]),
+                                            voxel_coord(p.z, sc.vs[2], sc.dims[2]), sc.tiled,
+                                            sc.dims[0], sc.dims[1], sc.nt0, sc.nt1);
+        };
+        const int vid = voxel(s);
+        const int st = __ldg(vstart + vid), c = __ldg(vcount + vid);
+        // the slot in its voxel's range, the range inside the scene; the slot before
+        // it in the same voxel; and the range's last slot, seen from its first
+        bool ok = s >= st && s - st < c && st >= sc.p_begin && c <= sc.p_begin + sc.p_count - st;
+        if (ok) ok = s > st ? voxel(s - 1) == vid : voxel(st + c - 1) == vid;
+        if (!ok) {
+            atomicOr(bad, 1);
+        } else if ((s - st) % kTaskRun == 0) {
+            tasks[atomicAdd(task_count, 1)] = make_int2(vid, s);
+            if (room.limit && sc.cap > kListCap && vid != sc.v_begin + sc.v_count) {
+                // as many voxels' particles within reach as the sphere is voxels large
+                const float one = fminf((float)c * (4.18879f * sc.h * sc.h * sc.h /
+                                                    (sc.vs[0] * sc.vs[1] * sc.vs[2])),
+                                        (float)sc.cap);
+                if (one > (float)kListCap)      // 32 of them fit 32 bits
+                    entries = (unsigned)(fminf(one, 4.0e6f) * (float)min(kTaskRun, st + c - s));
+            }
+        }
+    }
+    if (room.limit) {
+        // the last block to come by compares the sum
+        entries = __reduce_add_sync(0xffffffffu, entries);
+        if ((threadIdx.x & 31) == 0 && entries) {
+            atomicAdd(room.entries, (unsigned long long)entries);
+            __threadfence();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(room.blocks, 1) == (int)gridDim.x - 1 &&
+            atomicAdd(room.entries, 0ull) > room.limit)
+            atomicOr(bad, 1);
+    }
 }
 
 // Velocities of a state loaded in original particle order (scene offset + id)
@@ -1082,10 +1107,11 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
 
 cudaError_t launch_stage_tasks(const Launch& L, const float4* pos, const int32_t* vstart,
                                const int32_t* vcount, int2* tasks, int32_t* task_count,
-                               int32_t* bad) {
+                               int32_t* bad, StageRoom room) {
     if (L.n == 0) return cudaSuccess;
     k_stage_tasks<<<blocks_for(L.n), kBlock, 0, L.stream>>>(L.scenes, L.pbegin, L.n_scenes, L.n, pos,
-                                                            vstart, vcount, tasks, task_count, bad);
+                                                            vstart, vcount, tasks, task_count, bad,
+                                                            room);
     return cudaGetLastError();
 }
 
