@@ -96,8 +96,8 @@ constexpr int kHostEvents = kHostOrganizedEvent + 1;
 // device counters in big_count: big voxels, density tasks, tasks taken, then the
 // deferred particles of the whole force pass and of each host-entry range,
 // then the tasks of the second task list and those of it taken
-constexpr int kTcCounter = 4 + (kHostRanges > kPipeRanges ? kHostRanges : kPipeRanges);
-constexpr int kCounters = kTcCounter + 2;
+constexpr int kDenseCounter = 4 + (kHostRanges > kPipeRanges ? kHostRanges : kPipeRanges);
+constexpr int kCounters = kDenseCounter + 2;
 constexpr size_t kCountersPad = 64;      // ints; what follows stays 128-byte aligned
 constexpr int kOverCounter = (int)kCountersPad - 2;   // 64-bit: units of the list pool taken
 static_assert(kCounters <= kOverCounter, "counters");
@@ -109,9 +109,6 @@ constexpr size_t kOverMax = (size_t)1 << 28;
 // are cleared by bandwidth, not by latency (24 boxes with 1.6 M entries: step
 // 56.5 us with one buffer, 54.3 with two; 48 with 2.5 M: 264.9 and 265.7)
 constexpr size_t kTwoCounts = (size_t)1 << 21;
-// contexts of sparse and dense scenes: voxels of at most this many particles go
-// to k_density_tc, the others to k_density_wc
-constexpr int kTcVoxel = 48;
 
 struct SphgbCtx {
     int device = 0;
@@ -126,6 +123,8 @@ struct SphgbCtx {
     bool any_pipe = false;
     bool pairs = false;        // density tasks of two voxels (TaskLists)
     bool uncapped = false;     // some scene's cap is beyond kListCap
+    bool dense_scene = false;  // some capped scene's table is row-major
+    int largest_scene = 0;     // particles
     std::vector<SceneDev> h_scenes;
     std::vector<int32_t> h_pbegin;
     SceneDev* d_scenes = nullptr;       // step layout
@@ -244,17 +243,29 @@ struct SphgbCtx {
     cudaEvent_t pipe_ev[3 + kPipeRanges] = {};
     std::map<int, cudaGraphExec_t> graphs;
 
-    // Which density pass takes the step's tasks: k_density_tc those of sparse
-    // scenes (the tiled ones: 1.00 ms against 1.15 with k_density_wc on the
-    // 4,194,304-particle box, 73 against 90 us at 262,144) and of scenes
-    // without a cap (27 us against 330 at 32,768, where k_density_wc walks one
-    // thread per particle); k_density_wc those of dense scenes, where its homes
-    // skip voxels one by one (203 against 256 us on the 262,144-particle pipe).
-    // Contexts of both kinds split their tasks by voxel and run both.
-    enum DensityPass { kPassTc, kPassWc, kPassBoth };
-    DensityPass density_pass() const {
-        if (layout == 1 || uncapped) return kPassTc;
-        return layout == 2 ? kPassBoth : kPassWc;
+    // Which density pass takes the step's tasks: k_density_tc those of contexts
+    // with a sparse scene (the tiled ones: 0.94 ms against 1.15 with k_density_wc on
+    // the 4,194,304-particle box, 71 against 90 us at 262,144) or one without a
+    // cap (27 us against 330 at 32,768, where k_density_wc walks one thread per
+    // particle); k_density_wc those of the others (203 against 256 us on the
+    // 262,144-particle pipe).
+    bool tc() const { return layout != 0 || uncapped; }
+    // From how many particles on a voxel's tasks are listed apart in such a context
+    // (TaskLists), for k_density_wc: its homes skip voxels one by one and stop
+    // at their cap early, where k_density_tc keeps a batch as soon as one home
+    // needs it.  0: never.  Contexts with a dense capped scene (row-major table)
+    // split at 64: 230,000 particles at 133 per voxel beside an uncapped scene,
+    // step 319 -> 288 us (305 at 96: a few voxels stay behind, and their tasks
+    // are long), 262,144 in a pipe beside one 595 -> 547; 164,000 at 40 per voxel,
+    // of which few go, 173 -> 191 (176 at 96).  Other scenes may fill voxels as they run (a fluid that
+    // collects in part of its box): 1,000,000 particles at 1000 per voxel in a
+    // tiled table, step 2757 us, 1921 split at 192; at 400 1868 and 1457; at 133
+    // 1050 either way.  The second launch takes 1.1 us of every step, 1 % and more
+    // of that of 262,144 particles and fewer: those stay with k_density_tc
+    // (120,000 at 400 per voxel 348 us, 277 split; at 133 205 and 192).
+    int dense_from() const {
+        if (!tc() || density_variant != SPHGB_DENSITY_WARP) return 0;
+        return dense_scene ? 64 : largest_scene > (1 << 18) ? 192 : 0;
     }
     // the step's neighbour lists: with the pool when k_density_tc writes them all
     NbrList step_nbr() const {
@@ -278,15 +289,15 @@ struct SphgbCtx {
         TaskLists t;
         t.list = tasks;
         t.count = big_count + 1;
-        if (density_pass() == kPassBoth) {
-            t.tc_last = tasks + (n - 1);
-            t.tc_count = big_count + kTcCounter;
-            t.tc_max = kTcVoxel;
+        if ((t.dense_from = dense_from()) > 0) {
+            t.dense_last = tasks + (n - 1);
+            t.dense_count = big_count + kDenseCounter;
+            if (uncapped) t.scenes = d_scenes;
         }
         // With fewer particles than lanes at work every voxel has a warp of its own
         // at once, and a pair takes longer (8,192 particles: step 27.3 us without,
         // 27.5 with pairs; 15,294 in 6 boxes: 39.0 -> 34.2).
-        t.tc_next = density_variant == SPHGB_DENSITY_WARP && density_pass() == kPassTc;
+        t.tc_next = density_variant == SPHGB_DENSITY_WARP && tc();
         if (pairs && density_variant == SPHGB_DENSITY_WARP)
             t.pair_max = n > 64 * device_sm_count() ? kTaskRun : 0;
         return t;
@@ -956,12 +967,11 @@ int stage_lists(SphgbCtx* c, const StageScope& scope, const Launch& L, const flo
         room.blocks = l.words + 3;
     }
     SPHGB_CUDA(launch_stage_tasks(L, pos, vstart, vcount, l.tasks, l.words, bad, room));
-    // dense scenes: see density_pass
-    if (c->density_pass() == SphgbCtx::kPassWc)
-        SPHGB_CUDA(launch_density_wc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks,
+    if (!c->tc())
+        SPHGB_CUDA(launch_density_wc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks, 1,
                                      l.words, l.words + 1));
     else
-        SPHGB_CUDA(launch_density_tc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks, 1,
+        SPHGB_CUDA(launch_density_tc(L, pos, nullptr, vstart, vcount, rho, nullptr, out, l.tasks,
                                      l.words, l.words + 1, c->uncapped));
     return SPHGB_OK;
 }
@@ -1011,18 +1021,18 @@ int enqueue_step(SphgbCtx* c, cudaStream_t st, cudaEvent_t* ev = nullptr,
     if (organized) SPHGB_CUDA(cudaEventRecord(organized, st));
     const NbrList nbr = c->step_nbr();
     if (warp) {
-        const SphgbCtx::DensityPass pass = c->density_pass();
-        if (pass == SphgbCtx::kPassTc)
+        if (c->tc()) {
             SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                         nbr, lists.list, 1, lists.count, c->big_count + 2,
+                                         nbr, lists.list, lists.count, c->big_count + 2,
                                          c->uncapped));
-        else
+            if (lists.dense_from)
+                SPHGB_CUDA(launch_density_wc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
+                                             nbr, lists.dense_last, -1, lists.dense_count,
+                                             lists.dense_count + 1));
+        } else {
             SPHGB_CUDA(launch_density_wc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                         nbr, lists.list, lists.count, c->big_count + 2));
-        if (pass == SphgbCtx::kPassBoth)
-            SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
-                                         nbr, lists.tc_last, -1, lists.tc_count,
-                                         lists.tc_count + 1, false));
+                                         nbr, lists.list, 1, lists.count, c->big_count + 2));
+        }
     } else
         SPHGB_CUDA(launch_density(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
                                   nbr));
@@ -1192,8 +1202,13 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
     c->n_pipe_rows = n_pipe_rows_total;
     c->n_chunks = (int)chunks.size();
     c->any_pipe = any_pipe;
-    c->uncapped = false;
-    for (const SceneDev& d : c->h_scenes) c->uncapped |= d.cap > kListCap;
+    c->uncapped = c->dense_scene = false;
+    c->largest_scene = 0;
+    for (const SceneDev& d : c->h_scenes) {
+        c->largest_scene = std::max(c->largest_scene, (int)d.p_count);
+        c->uncapped |= d.cap > kListCap;
+        c->dense_scene |= d.cap <= kListCap && !d.tiled;
+    }
     if (c->uncapped && N > 0) {
         c->over_units = std::min(N * kOverPerParticle, kOverMax);
         // without the pool the force pass walks again: slower, the same results
@@ -1741,13 +1756,13 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
             const int b = b_density;
             const VelRows vr = b < kPipeGathered ? VelRows{} : vrows;
             if (b == kPipeGathered) SPHGB_CUDA(cudaStreamWaitEvent(st, e_vel, 0));
-            if (c->density_pass() == SphgbCtx::kPassTc)
+            if (c->tc())
                 SPHGB_CUDA(launch_density_tc(L, c->posB, nullptr, c->vstart, c->vcount, c->rho,
-                                             c->fin, c->nbr, c->tasks_b, 1, pi + b,
-                                             pi + 2 * kPipeK + b, false, pi + 4 * kPipeK + b, vr));
+                                             c->fin, c->nbr, c->tasks_b, pi + b, pi + 2 * kPipeK + b,
+                                             false, pi + 4 * kPipeK + b, vr));
             else
                 SPHGB_CUDA(launch_density_wc(L, c->posB, nullptr, c->vstart, c->vcount, c->rho,
-                                             c->fin, c->nbr, c->tasks_b, pi + b,
+                                             c->fin, c->nbr, c->tasks_b, 1, pi + b,
                                              pi + 2 * kPipeK + b, pi + 4 * kPipeK + b, vr));
             if (b >= kPipeGathered) continue;
             if (b == 0) SPHGB_CUDA(cudaStreamWaitEvent(st, e_vel, 0));

@@ -399,7 +399,7 @@ __device__ __forceinline__ uint32_t tc_sum(TcCursor& C, int n, uint32_t row, uin
 }
 
 // kLayout: 0 every scene's voxel table row-major, 1 every one tiled, 2 per scene.
-// Task t is at tasks[t * dir].  kUncapped: some scene's cap is beyond kListCap.
+// kUncapped: some scene's cap is beyond kListCap.
 // kGather: the task's velocities too, from FP64 rows (vrows).
 template <int kLayout, bool kUncapped, bool kGather>
 __global__ void __launch_bounds__(kTcWarps * 32, 6)
@@ -408,7 +408,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
              const float4* __restrict__ vel, const int32_t* __restrict__ vstart,
              const int32_t* __restrict__ vcount, float* __restrict__ rho,
              float4* __restrict__ fin, NbrList nbr,
-             const int2* __restrict__ tasks, int dir, const int32_t* __restrict__ task_count,
+             const int2* __restrict__ tasks, const int32_t* __restrict__ task_count,
              int32_t* __restrict__ task_next, const int32_t* __restrict__ task_offset,
              VelRows vrows) {
     __shared__ TcShared sh[kTcWarps];
@@ -430,7 +430,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     for (;;) {
         const int t = __shfl_sync(full, next, 0);    // uniform, also to the compiler
         if (t >= n_tasks) break;
-        const int2 task = after_wait(tasks)[t * dir];
+        const int2 task = after_wait(tasks)[t];
         if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
         // a pair task (see TaskLists) has its first voxel's index complemented
         const bool pair = kLayout == 1 && !kGather && task.x < 0;
@@ -735,7 +735,7 @@ k_density_tc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
 
 cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
-                              float4* fin, NbrList nbr, const int2* tasks, int dir,
+                              float4* fin, NbrList nbr, const int2* tasks,
                               const int32_t* task_count, int32_t* task_next, bool uncapped,
                               const int32_t* task_offset, VelRows vrows) {
     if (L.n == 0) return cudaSuccess;
@@ -752,7 +752,7 @@ cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* 
                                  : L.layout == 2 ? k_density_tc<2, false, false>
                                                  : k_density_tc<0, false, false>);
     return launch_chained(kernel, blocks, kTcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
-                          L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, dir, task_count,
+                          L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, task_count,
                           task_next, task_offset, vrows);
 }
 

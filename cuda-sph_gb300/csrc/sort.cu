@@ -423,9 +423,11 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
                 mine = !(vid & 16);       // the even voxel's first particle lists the pair
             }
         }
+        bool dense = tasks.dense_from && c >= tasks.dense_from;
+        if (dense && tasks.scenes) dense = tasks.scenes[scene_of(s, pbegin, n_scenes)].cap <= kListCap;
         if (!mine) {
-        } else if (c <= tasks.tc_max)
-            tasks.tc_last[-atomicAdd(tasks.tc_count, 1)] = make_int2(vid, d);
+        } else if (dense)
+            tasks.dense_last[-atomicAdd(tasks.dense_count, 1)] = make_int2(vid, d);
         else
             tasks.list[atomicAdd(tasks.count, 1)] = make_int2(first, d);
     }

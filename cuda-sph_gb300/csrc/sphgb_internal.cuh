@@ -705,10 +705,10 @@ cudaError_t launch_sort_big(const Launch& L, const int32_t* big_list, const int3
 // Density tasks: one (voxel, first slot) entry per run of up to kTaskRun
 // sorted slots of a voxel; a warp of the density pass takes one task at a time.
 constexpr int kTaskRun = 16;
-// A task in a voxel of at most tc_max particles goes to the list that ends at
-// tc_last (entry t at tc_last[-t]); the others to the list from `list` on.
-// Both share one array: there are no more tasks than particles.  list null:
-// no tasks.
+// Tasks in voxels of at least dense_from particles, of capped scenes (asked when
+// `scenes` is given), go to the list that ends at dense_last (entry t at
+// dense_last[-t]); the others to the list from `list` on.  Both share one
+// array: there are no more tasks than particles.  list null: no tasks.
 //
 // Pairs (contexts whose scenes are all tiled, with voxels at least h deep): two
 // voxels that are neighbours in z, 2k and 2k + 1, of at most pair_max <= kTaskRun
@@ -720,9 +720,10 @@ constexpr int kTaskRun = 16;
 struct TaskLists {
     int2* list = nullptr;
     int32_t* count = nullptr;
-    int2* tc_last = nullptr;
-    int32_t* tc_count = nullptr;
-    int tc_max = 0;      // one list
+    int2* dense_last = nullptr;
+    int32_t* dense_count = nullptr;
+    int dense_from = 0;  // 0: one list
+    const SceneDev* scenes = nullptr;   // null: every scene is capped
     int pair_max = 0;    // 0: none
     bool tc_next = false;    // k_density_tc is the kernel after the rank-gather
 };
@@ -758,19 +759,19 @@ cudaError_t launch_stage_tasks(const Launch& L, const float4* pos, const int32_t
                                const int32_t* vcount, int2* tasks, int32_t* task_count,
                                int32_t* bad, StageRoom room = StageRoom{});
 // the step's density pass: one warp per task (<= kTaskRun particles of one voxel);
-// task_next: a zeroed counter from which the warps take the tasks
+// task t is at tasks[t * dir]; task_next: a zeroed counter from which the warps
+// take the tasks
 // task_offset (optional, device): the tasks start at tasks[*task_offset] (one
 // bucket of a bucketed list)
 cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
-                              float4* fin, NbrList nbr, const int2* tasks,
+                              float4* fin, NbrList nbr, const int2* tasks, int dir,
                               const int32_t* task_count, int32_t* task_next,
                               const int32_t* task_offset = nullptr, VelRows vrows = VelRows{});
-// the same on the tensor cores; task t is at tasks[t * dir]; uncapped: some
-// scene's cap is beyond kListCap
+// the same on the tensor cores (dir 1); uncapped: some scene's cap is beyond kListCap
 cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
-                              float4* fin, NbrList nbr, const int2* tasks, int dir,
+                              float4* fin, NbrList nbr, const int2* tasks,
                               const int32_t* task_count, int32_t* task_next, bool uncapped,
                               const int32_t* task_offset = nullptr, VelRows vrows = VelRows{});
 // k_gather_vel over the slots of a bucket of density tasks

@@ -241,7 +241,8 @@ __device__ __forceinline__ void wc_candidates(WcShared& S, int& cnt, bool home, 
 }
 
 // kLayout: 0 every scene's voxel table row-major, 1 every one tiled, 2 per scene.
-// kGather: the task's velocities too, from FP64 rows (vrows).
+// Task t is at tasks[t * dir].  kGather: the task's velocities too, from FP64 rows
+// (vrows).
 template <int kLayout, bool kGather>
 __global__ void __launch_bounds__(kWcWarps * 32, 4)
 k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin,
@@ -249,7 +250,7 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
              const float4* __restrict__ vel, const int32_t* __restrict__ vstart,
              const int32_t* __restrict__ vcount, float* __restrict__ rho,
              float4* __restrict__ fin, NbrList nbr,
-             const int2* __restrict__ tasks, const int32_t* __restrict__ task_count,
+             const int2* __restrict__ tasks, int dir, const int32_t* __restrict__ task_count,
              int32_t* __restrict__ task_next, const int32_t* __restrict__ task_offset,
              VelRows vrows) {
     __shared__ WcShared sh[kWcWarps];
@@ -269,7 +270,7 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
     for (;;) {
         const int t = __shfl_sync(full, next, 0);    // uniform, also to the compiler
         if (t >= n_tasks) break;
-        const int2 task = after_wait(tasks)[t];
+        const int2 task = after_wait(tasks)[t * dir];
         const int vid = task.x, d0 = task.y;
         const SceneDev& sc = scenes[scene_of_warp(d0, pbegin, n_scenes)];
         const int vst = __ldg(vstart + vid), vc = __ldg(vcount + vid);
@@ -1081,7 +1082,7 @@ cudaError_t launch_density(const Launch& L, const float4* pos, const float4* vel
 
 cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* vel,
                               const int32_t* vstart, const int32_t* vcount, float* rho,
-                              float4* fin, NbrList nbr, const int2* tasks,
+                              float4* fin, NbrList nbr, const int2* tasks, int dir,
                               const int32_t* task_count, int32_t* task_next,
                               const int32_t* task_offset, VelRows vrows) {
     if (L.n == 0) return cudaSuccess;
@@ -1101,7 +1102,7 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
                          : L.layout == 2 ? k_density_wc<2, false>
                                          : k_density_wc<0, false>);
     return launch_chained(kernel, blocks, kWcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
-                          L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, task_count, task_next,
+                          L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, dir, task_count, task_next,
                           task_offset, vrows);
 }
 
