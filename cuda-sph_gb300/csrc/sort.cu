@@ -282,20 +282,17 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
         quarter_sync(quarter);
         for (int i = t; i < c; i += kQuarter) {
             const int32_t p = sq[i];
-            // the warp's own 32 ids lie between those that come before all of
-            // its ids and those that come after: equal ids keep their order
-            const int own = i & ~31, after = min(own + 32, c4);
-            int r = 0;
-            for (int k = 0; k < own; k += 4) {
+            // equal ids keep their order: those before the warp's own 32 count, and
+            // those of lower lanes
+            const int own = i & ~31;
+            const unsigned live = c - own >= 32 ? 0xffffffffu : (1u << (c - own)) - 1u;
+            int r = __popc(__match_any_sync(live, p) & ((1u << (i & 31)) - 1u));
+            int k = 0;
+            for (; k < own; k += 4) {
                 const int4 q = *reinterpret_cast<const int4*>(sq + k);
                 r += (q.x <= p) + (q.y <= p) + (q.z <= p) + (q.w <= p);
             }
-            for (int k = own; k < after; k += 4) {
-                const int4 q = *reinterpret_cast<const int4*>(sq + k);
-                r += (q.x < p || (q.x == p && k < i)) + (q.y < p || (q.y == p && k + 1 < i)) +
-                     (q.z < p || (q.z == p && k + 2 < i)) + (q.w < p || (q.w == p && k + 3 < i));
-            }
-            for (int k = after; k < c4; k += 4) {
+            for (; k < c4; k += 4) {
                 const int4 q = *reinterpret_cast<const int4*>(sq + k);
                 r += (q.x < p) + (q.y < p) + (q.z < p) + (q.w < p);
             }
