@@ -101,8 +101,9 @@ constexpr int kCounters = kDenseCounter + 2;
 constexpr size_t kCountersPad = 64;      // ints; what follows stays 128-byte aligned
 constexpr int kOverCounter = (int)kCountersPad - 2;   // 64-bit: units of the list pool taken
 static_assert(kCounters <= kOverCounter, "counters");
-// pool of the lists that do not fit their rows (scenes without a cap): 128
-// entries per particle, 8 GB at most
+// pool of the lists that do not fit their rows: units of 8 entries, 128 entries (512
+// bytes) per particle of the scenes with a cap beyond kListCap or none, 8.6 GB
+// at most; the stage calls have a second one like it (stage_lists)
 constexpr size_t kOverPerParticle = 128 / 8;
 constexpr size_t kOverMax = (size_t)1 << 28;
 // voxel tables of at most this many entries have two count buffers; larger ones
@@ -943,7 +944,7 @@ int stage_lists(SphgbCtx* c, const StageScope& scope, const Launch& L, const flo
         cudaThreadExchangeStreamCaptureMode(&mode);
         int rc = dalloc(&l.tasks, N);
         if (!rc) rc = dalloc(&l.words, head + (kListCap + 1) * N + 8);
-        if (!rc && c->uncapped) rc = dalloc(&l.over, 8 * (size_t)std::min(N * kOverPerParticle, kOverMax));
+        if (!rc && c->uncapped) rc = dalloc(&l.over, 8 * (size_t)c->over_units);
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (rc) {
             free_lists(c);
@@ -961,7 +962,7 @@ int stage_lists(SphgbCtx* c, const StageScope& scope, const Launch& L, const flo
     if (c->uncapped && !rho) {      // the density call reads no list
         out.over = l.over;
         out.over_used = reinterpret_cast<unsigned long long*>(l.words + kOverCounter);
-        out.over_units = std::min(N * kOverPerParticle, kOverMax);
+        out.over_units = c->over_units;
         room.limit = 8 * out.over_units;
         room.entries = reinterpret_cast<unsigned long long*>(l.words + kOverCounter - 2);
         room.blocks = l.words + 3;
@@ -1209,10 +1210,23 @@ int configure(SphgbCtx* c, const SphgbSceneParams* scenes, int n_scenes,
         c->uncapped |= d.cap > kListCap;
         c->dense_scene |= d.cap <= kListCap && !d.tiled;
     }
-    if (c->uncapped && N > 0) {
-        c->over_units = std::min(N * kOverPerParticle, kOverMax);
-        // without the pool the force pass walks again: slower, the same results
-        if (ensure(&c->over, k.over, 8 * (size_t)c->over_units) != SPHGB_OK) g_last_error.clear();
+    {
+        size_t listed = 0;      // particles of such scenes
+        for (const SceneDev& d : c->h_scenes)
+            if (d.cap > kListCap) listed += (size_t)d.p_count;
+        c->over_units = std::min(listed * kOverPerParticle, kOverMax);
+        // as large as it is used, and given back with the last such scene.
+        // Without the pool the force pass walks again: slower, the same results.
+        const size_t need = 8 * (size_t)c->over_units;
+        if (c->over && (need == 0 || k.over < need)) {
+            cudaFree(c->over);
+            c->over = nullptr;
+            k.over = 0;
+        }
+        if (need > 0 && !c->over) {
+            if (dalloc(&c->over, need) == SPHGB_OK) k.over = need;
+            else g_last_error.clear();
+        }
     }
     // the caller binds (new) state and outputs for the new layout
     c->bound = false;

@@ -43,10 +43,13 @@ from .device import SceneBatch, SceneSpec
 # HBM bytes per particle for a scene resident in the batch: bound state
 # (pos, vel 16 B each, rho, pid 4 B), the step's sorted copies (36 B), ids and
 # ranks (12 B), force inputs (32 B), neighbour list (132 B), density tasks (8 B),
-# export staging (56 B) and the FP64 accumulator (48 B both buffers, pipe scenes)
+# export staging (56 B) and the FP64 accumulator (48 B both buffers, pipe scenes);
+# scenes with a cap beyond 32 neighbours, or none, share a pool of long lists.
+# Per voxel: its start and two count buffers.
 BYTES_PER_PARTICLE = 40 + 36 + 12 + 32 + 132 + 8 + 56
 BYTES_PER_PIPE_PARTICLE = 48
-BYTES_PER_VOXEL = 8
+BYTES_PER_LONG_LIST_PARTICLE = 512
+BYTES_PER_VOXEL = 12
 
 
 def footprint(spec: SceneSpec) -> int:
@@ -54,6 +57,8 @@ def footprint(spec: SceneSpec) -> int:
     voxel = np.asarray(spec.params.voxel_size, dtype=np.float64)
     voxels = int(np.prod(np.ceil(space / voxel))) + 1
     per = BYTES_PER_PARTICLE + (BYTES_PER_PIPE_PARTICLE if spec.mode == 'PIPE' else 0)
+    if not 0 < spec.constants.max_neighbours <= 32:
+        per += BYTES_PER_LONG_LIST_PARTICLE
     return spec.n * per + voxels * BYTES_PER_VOXEL
 
 
