@@ -241,7 +241,7 @@ struct SphgbCtx {
     int32_t* h_pipe = nullptr;
     size_t cap_tasks_b = 0, cap_vbucket = 0;
     cudaStream_t host_stream4 = nullptr;
-    cudaEvent_t pipe_ev[3 + kPipeRanges] = {};
+    cudaEvent_t pipe_ev[2 + kPipeRanges] = {};
     std::map<int, cudaGraphExec_t> graphs;
 
     // Which density pass takes the step's tasks: k_density_tc those of contexts
@@ -1719,8 +1719,8 @@ int host_step_pipelined(SphgbCtx* c, cudaEvent_t e_vel, double* sp, double* sv, 
                         double* h_pos_out, double* h_vel_out, double* h_rho_out) {
     const size_t N = (size_t)c->n;
     cudaStream_t st = c->host_stream, st4 = c->host_stream4;
-    cudaEvent_t e_bk = c->pipe_ev[1], e_dep = c->pipe_ev[2];
-    cudaEvent_t* e_range = c->pipe_ev + 3;
+    cudaEvent_t e_bk = c->pipe_ev[0], e_dep = c->pipe_ev[1];
+    cudaEvent_t* e_range = c->pipe_ev + 2;
     const Launch L = c->launch(st);
     double* p64A = c->any_pipe ? c->pos64A : nullptr;
     double* p64B = c->any_pipe ? c->pos64B : nullptr;

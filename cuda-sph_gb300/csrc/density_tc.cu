@@ -743,8 +743,9 @@ cudaError_t launch_density_tc(const Launch& L, const float4* pos, const float4* 
     // take tasks in turn; small scenes get about a warp per task, so that the
     // tasks spread over the SMs (a task's latency is most of their pass)
     const int blocks = std::min((L.n + 8 * kTcWarps - 1) / (8 * kTcWarps), device_sm_count() * 6);
-    // the velocity gather is for one capped scene (the pipelined host order)
-    auto kernel = vrows.vel64 ? (L.layout == 1 ? k_density_tc<1, false, true> : k_density_tc<0, false, true>)
+    // the velocity gather is for one capped sparse scene (the pipelined host order)
+    if (vrows.vel64 && (L.layout != 1 || uncapped)) return cudaErrorInvalidValue;
+    auto kernel = vrows.vel64 ? k_density_tc<1, false, true>
                   : uncapped  ? (L.layout == 1   ? k_density_tc<1, true, false>
                                  : L.layout == 2 ? k_density_tc<2, true, false>
                                                  : k_density_tc<0, true, false>)

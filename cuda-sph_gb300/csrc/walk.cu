@@ -107,8 +107,8 @@ k_density(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegi
                          &s_list[0][threadIdx.x], kBlock);
 }
 
-// Warp-cooperative density pass of the step of dense scenes, and of the
-// pipelined host order (sparse scenes: density_tc.cu).  One warp per task: up to
+// Warp-cooperative density pass of the capped tasks of dense scenes and voxels
+// (sparse and uncapped ones: density_tc.cu).  One warp per task: up to
 // kTaskRun particles of one voxel (tasks listed by the rank-gather).  The 27
 // walk voxels of that voxel are laid end to end in walk order; each batch of
 // 96 candidates is loaded coalesced, three per lane (a candidate's slot found
@@ -280,22 +280,6 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
         const float4 pi = home ? __ldg(pos + s) : make_float4(0.f, 0.f, 0.f, 0.f);
         const int local = vid - sc.v_begin;
         const int cap = sc.cap;
-        if (local == sc.v_count || cap > kListCap) {
-            // overflow bucket (non-finite positions) or a cap beyond the shared
-            // list: thread-private walk per particle
-            if (home) {   // S.e[lane] serves as its row buffer
-                density_one<kLayout>(s, pi, sc, pos, vel, vstart, vcount, n, rho, fin, nbr,
-                                     &S.e[lane][0].x, 1);
-                if (kGather) {
-                    const float4 v = vel_row(vrows, s, pbegin, n_scenes);
-                    vrows.vel_out[s] = v;
-                    fin[2 * s + 1] = make_float4(v.x, v.y, v.z, 1.0f / rho[s]);
-                }
-            }
-            if (lane == 0) next = n_warps + atomicAdd(task_next, 1);
-            __syncwarp();
-            continue;
-        }
         if (home) S.home[lane] = pi;
         // the 27 walk voxels (voxel_kernels.py:46-61 order), from the table coords
         const int tiled = kLayout == 2 ? sc.tiled : kLayout;
@@ -330,7 +314,9 @@ k_density_wc(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pb
             const int v = __shfl_up_sync(full, incl, o);
             if (lane >= o) incl += v;
         }
-        const int M = __shfl_sync(full, incl, 26);   // candidates in the whole walk
+        // candidates in the whole walk; none for the overflow entry, whose
+        // particles (non-finite positions) have no neighbours
+        const int M = local == sc.v_count ? 0 : __shfl_sync(full, incl, 26);
         // Candidate q (walk order) lies in the non-empty walk voxel with the
         // largest first index P_k <= q; its slot is q + (start_k - P_k).  Lane
         // k keeps P_k; S.off holds start_k - P_k by rank among the non-empty
@@ -1093,14 +1079,13 @@ cudaError_t launch_density_wc(const Launch& L, const float4* pos, const float4* 
     int blocks = (L.n + 8 * kWcWarps - 1) / (8 * kWcWarps);
     const int top = device_sm_count() * 4;
     if (blocks > top) blocks = top;
-    // the velocity gather is its own instantiation: the step's kernel stays as it is
-    auto kernel = vrows.vel64
-                      ? (L.layout == 1   ? k_density_wc<1, true>
-                         : L.layout == 2 ? k_density_wc<2, true>
-                                         : k_density_wc<0, true>)
-                      : (L.layout == 1   ? k_density_wc<1, false>
-                         : L.layout == 2 ? k_density_wc<2, false>
-                                         : k_density_wc<0, false>);
+    // the velocity gather is its own instantiation: the step's kernel stays as it
+    // is.  It is for one dense scene (the pipelined host order).
+    if (vrows.vel64 && L.layout != 0) return cudaErrorInvalidValue;
+    auto kernel = vrows.vel64     ? k_density_wc<0, true>
+                  : L.layout == 1 ? k_density_wc<1, false>
+                  : L.layout == 2 ? k_density_wc<2, false>
+                                  : k_density_wc<0, false>;
     return launch_chained(kernel, blocks, kWcWarps * 32, L, L.scenes, L.pbegin, L.n_scenes,
                           L.n, pos, vel, vstart, vcount, rho, fin, nbr, tasks, dir, task_count, task_next,
                           task_offset, vrows);
