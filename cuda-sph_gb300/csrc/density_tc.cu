@@ -53,14 +53,20 @@ constexpr int kTcGroups = 2;                 // groups of 32 candidates per batc
 constexpr int kTcBatch = 32 * kTcGroups;
 constexpr int kTcChunk = 320;                // candidates held in shared memory
 constexpr int kTcWords = kTcChunk / 32;
-constexpr int kTcCullMin = 640;  // walks longer than this pass over unreachable batches
-constexpr int kTcBallot = 4;     // tasks of at most this many homes test with ballots
+// Walks longer than this pass over unreachable batches: two chunks and more.  At 320
+// the masks cost more than they save (4,194,304-particle box 0.967 ms, 0.940 so);
+// beyond 640, or never, within 1 % from 4 to 80 particles per voxel.
+constexpr int kTcCullMin = 640;
+// Tasks of at most this many homes test with ballots: 0.940 ms with 2 as with
+// 4, 0.973 with 8.
+constexpr int kTcBallot = 4;
 // Bound on |computed - exact| of (d^2 - h^2) / vs^2 for candidates of |u|^2 <=
 // kTcFar, homes of |u|^2 <= kTcHome and (h / vs)^2 <= kTcH2 (others are decided
 // by ballots): every partial sum is below 9 + 2 sqrt(9 * 1.6) + 2 < 32.  The FP32
 // rounding of u and |u|^2 gives 2^-17.4, the FP16 pairs 2^-17.4 over the products
 // and |u|^2, 17 accumulations truncated at 2^-19 each 2^-14.9: 2^-14.4 = 5e-5
-// together.
+// together.  (PTX gives mma's FP32 accumulation at least single precision and
+// leaves the rounding open: truncation of 24 bits is the worst it allows.)
 constexpr float kTcTol = 1.0e-4f;
 constexpr float kTcFar = 9.0f;    // |u|^2 within the walk: 3 * 1.5^2, pairs 2 * 1.5^2 + 2^2
 constexpr float kTcHome = 1.6f;   // 3 * 0.5^2, pairs 2 * 0.5^2 + 1

@@ -488,9 +488,8 @@ k_gather_vel(const int32_t* __restrict__ pbegin, int n_scenes, int n,
 // entry): one thread per slot of the bucket's tasks (a task's run of at most
 // kTaskRun slots of one voxel), kTaskRun threads per task.  The velocities
 // come straight from the uploaded FP64 rows (original order), converted as
-// k_load_aos converts them: the float4 state buffer is the force pass's
-// output, which earlier force buckets are already writing (in slot order)
-// while later buckets gather.
+// k_load_aos converts them: no pass over the velocities stands between the
+// upload and the first bucket.
 __global__ void __launch_bounds__(kBlock)
 k_gather_vel_tasks(const int32_t* __restrict__ pbegin, int n_scenes, const int32_t* __restrict__ pid,
                    const int32_t* __restrict__ vstart, const int32_t* __restrict__ vcount,
@@ -727,7 +726,7 @@ k_forces(const SceneDev* __restrict__ scenes, const int32_t* __restrict__ pbegin
 // particles with every path.  The per-particle arithmetic is the same in all
 // three: the results are identical.
 constexpr int kForceAll = 0, kForceLean = 1, kForceRare = 2;
-// kForceRare grid: one block per SM (device_sm_count())
+// kForceRare grid: up to four blocks per SM (device_sm_count())
 
 // Which particles a force launch runs: every slot (kBySlot); the particles of
 // rows range.i0..i1 in original order, which also write the FP64 rows of the

@@ -260,7 +260,14 @@ int sphgb_ctx_set_checks(SphgbCtx* ctx, int enable);
  * checked mode was never enabled. */
 int sphgb_ctx_check_word(SphgbCtx* ctx, uint32_t* h_word, int clear, void* stream);
 
-/* ---- stages (each launches the same kernels sphgb_ctx_step uses) ------- */
+/* ---- stages (each launches the same kernels sphgb_ctx_step uses) -------
+ * sphgb_density, sphgb_forces and sphgb_integrate share force records and
+ * neighbour lists of the context: each call waits on the device for the one
+ * before it, also when that was on another stream (not under stream capture).
+ * The lists are allocated by the first such call: 140 bytes per particle, and
+ * 512 more per particle of scenes with a cap beyond 32 or none; without memory
+ * for them, and under capture, the calls walk the voxels instead (slower, the
+ * same results). */
 
 /* assign_voxels_to_particles_kernel (voxel_kernels.py:89-105): voxel id of
  * each particle (ceil dims; coordinates clamped to the table).  A particle
@@ -268,9 +275,11 @@ int sphgb_ctx_check_word(SphgbCtx* ctx, uint32_t* h_word, int clear, void* strea
  * entry, the last entry of the scene's voxel table. */
 int sphgb_assign_voxels(SphgbCtx* ctx, const float* d_pos, int32_t* d_voxel_out, void* stream);
 
-/* Voxel sort + voxel_begin (voxel_sph_strategy.py:65-107): stable counting
- * sort by (voxel id, particle id); particles of a scene's overflow entry
- * (non-finite coordinates, never walked) come last, in arrival order.  Reads state (d_pos, d_vel, d_pid) in any
+/* Voxel sort + voxel_begin (voxel_sph_strategy.py:65-107): counting sort by
+ * (voxel id, particle id), the ids of a voxel distinct (of particles with the
+ * same id one is kept, in the first of their slots; the others are left
+ * unwritten); particles of a scene's overflow entry (non-finite coordinates,
+ * never walked) come last, in arrival order.  Reads state (d_pos, d_vel, d_pid) in any
  * order, writes it voxel-sorted to the *_out buffers, and writes the voxel
  * table: d_voxel_start[v] (first sorted slot) and d_voxel_count[v]. */
 int sphgb_organize_voxels(SphgbCtx* ctx, const float* d_pos, const float* d_vel,
