@@ -3,8 +3,10 @@
 // A context (SphgbCtx) holds the scene descriptors, the pipe table and every
 // scratch buffer of the step; the caller owns the particle state and binds it.
 // The step enqueues, per time step:
-//   memset(voxel_count) -> hash+histogram -> scan -> scatter -> rank-gather
-//   -> density -> force+integrate+wall -> step counter
+//   memset(counts; a multi-step call's first step) -> hash+histogram -> scan
+//   -> scatter -> big-voxel sort -> rank-gather -> density (one or two kernels)
+//   -> force+integrate+wall -> deferred particles and step counter
+// (pipe scenes, checked and profiled steps: a step-counter kernel at the end),
 // which is VoxelSPHStrategy.compute_next_state (sim/src/sph/strategies/
 // abstract_sph_strategy.py:31-46, voxel_sph_strategy.py:20-116) without any
 // host round trip.
@@ -248,22 +250,24 @@ struct SphgbCtx {
     // with a sparse scene (the tiled ones: 0.94 ms against 1.15 with k_density_wc on
     // the 4,194,304-particle box, 71 against 90 us at 262,144) or one without a
     // cap (27 us against 330 at 32,768, where k_density_wc walks one thread per
-    // particle); k_density_wc those of the others (203 against 256 us on the
+    // particle); k_density_wc those of the others (195 against 256 us on the
     // 262,144-particle pipe).
     bool tc() const { return layout != 0 || uncapped; }
     // From how many particles on a voxel's tasks are listed apart in such a context
-    // (TaskLists), for k_density_wc: its homes skip voxels one by one and stop
-    // at their cap early, where k_density_tc keeps a batch as soon as one home
-    // needs it.  0: never.  Contexts with a dense capped scene (row-major table)
-    // split at 64: 230,000 particles at 133 per voxel beside an uncapped scene,
-    // step 319 -> 288 us (305 at 96: a few voxels stay behind, and their tasks
-    // are long), 262,144 in a pipe beside one 595 -> 547; 164,000 at 40 per voxel,
-    // of which few go, 173 -> 191 (176 at 96).  Other scenes may fill voxels as they run (a fluid that
-    // collects in part of its box): 1,000,000 particles at 1000 per voxel in a
-    // tiled table, step 2757 us, 1921 split at 192; at 400 1868 and 1457; at 133
-    // 1050 either way.  The second launch takes 1.1 us of every step, 1 % and more
-    // of that of 262,144 particles and fewer: those stay with k_density_tc
-    // (120,000 at 400 per voxel 348 us, 277 split; at 133 205 and 192).
+    // (TaskLists), for k_density_wc: its homes skip voxels one by one and stop at
+    // their cap early, where k_density_tc keeps a batch as soon as one home needs
+    // it.  0: never.
+    // Contexts with a dense capped scene (row-major table) split at 64: 230,000
+    // particles at 133 per voxel beside an uncapped scene, step 319 -> 288 us (305 at
+    // 96: a few voxels stay behind, and their tasks are long), 262,144 in a pipe
+    // beside one 595 -> 547; 164,000 at 40 per voxel, of which few go, 173 -> 191
+    // (176 at 96).
+    // Other scenes may fill voxels as they run (a fluid that collects in part of
+    // its box): 1,000,000 particles at 1000 per voxel in a tiled table, step 2757
+    // us, 1921 split at 192; at 400 1868 and 1457; at 133 1050 either way.  The
+    // second launch takes 1.1 us of every step, 1 % and more of that of 262,144
+    // particles and fewer: those stay with k_density_tc (120,000 at 400 per voxel
+    // 348 us, 277 split; at 133 205 and 192).
     int dense_from() const {
         if (!tc() || density_variant != SPHGB_DENSITY_WARP) return 0;
         return dense_scene ? 64 : largest_scene > (1 << 18) ? 192 : 0;
@@ -290,7 +294,8 @@ struct SphgbCtx {
         TaskLists t;
         t.list = tasks;
         t.count = big_count + 1;
-        if ((t.dense_from = dense_from()) > 0) {
+        if (const int from = dense_from()) {
+            t.dense_from = from;
             t.dense_last = tasks + (n - 1);
             t.dense_count = big_count + kDenseCounter;
             if (uncapped) t.scenes = d_scenes;
@@ -298,7 +303,7 @@ struct SphgbCtx {
         // With fewer particles than lanes at work every voxel has a warp of its own
         // at once, and a pair takes longer (8,192 particles: step 27.3 us without,
         // 27.5 with pairs; 15,294 in 6 boxes: 39.0 -> 34.2).
-        t.tc_next = density_variant == SPHGB_DENSITY_WARP && tc();
+        t.tc_next = density_variant == SPHGB_DENSITY_WARP && tc() && !dense_scene;
         if (pairs && density_variant == SPHGB_DENSITY_WARP)
             t.pair_max = n > 64 * device_sm_count() ? kTaskRun : 0;
         return t;
@@ -474,9 +479,11 @@ int build_scene(const SphgbSceneParams& p, int n_pipe_rows_total, SceneDev& d,
     return SPHGB_OK;
 }
 
-// Rows of 3 doubles go through shared memory, so that a warp's accesses are
-// whole lines: they may go over the host link (host_entry's direct order), and
-// on the device a thread's own 24 bytes touch three times the sectors.
+// Rows of 3 doubles through shared memory, so that a warp's accesses are whole
+// lines: rows that go over the host link (host_entry's direct order), and the
+// store's on the device, where a thread's own 24 bytes touch three times the
+// sectors.  Device loads stay the thread's own, which hit L1 (4,194,304 rows 67
+// us, 92 through shared memory).
 __device__ __forceinline__ void load_rows(double* buf, const double* __restrict__ src, int i, int m) {
     for (int k = threadIdx.x; k < 3 * m; k += kBlock) buf[k] = src[3 * (size_t)i + k];
 }
@@ -1026,7 +1033,7 @@ int enqueue_step(SphgbCtx* c, cudaStream_t st, cudaEvent_t* ev = nullptr,
             SPHGB_CUDA(launch_density_tc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
                                          nbr, lists.list, lists.count, c->big_count + 2,
                                          c->uncapped));
-            if (lists.dense_from)
+            if (lists.dense_last)
                 SPHGB_CUDA(launch_density_wc(L, c->posB, vel_s, c->vstart, c->vcount, c->rho, c->fin,
                                              nbr, lists.dense_last, -1, lists.dense_count,
                                              lists.dense_count + 1));
@@ -1506,7 +1513,8 @@ constexpr int kPipeGathered = 1;
 
 // Range r of the original indices is [b[r], b[r + 1]).  The last ranges are
 // smaller: the force buckets and downloads that must wait for the end of the
-// density pass are short.  Relative sizes of the ranges:
+// density pass are short (4,194,304 particles 2.85 ms per call; ranges of one
+// size 2.88, a last third of 8, 2 and 1 2.88).  Relative sizes of the ranges:
 constexpr int kPipeWeight[kPipeK] = {4, 4, 4, 4, 4, 2, 1};
 struct PipeBounds {
     int32_t b[kPipeK + 1];

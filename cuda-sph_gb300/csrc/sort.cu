@@ -14,9 +14,9 @@
 //      order exactly, independent of atomic arrival order and of the input
 //      order of the state.
 // Voxels with more than kBigVoxel members (dense clusters, the overflow bucket
-// of non-finite particles) have their member ids sorted by one block each
-// between 3 and 4, and the rank is a binary search, so the pass stays
-// O(n log n) however the particles cluster.
+// of non-finite particles) have their member ids sorted between 3 and 4, by a
+// quarter of a block each or a whole one, and the rank is a binary search, so
+// the pass stays O(n log n) however the particles cluster.
 #include <algorithm>
 #include <climits>
 
@@ -342,8 +342,9 @@ k_sort_big(const int32_t* __restrict__ big_list, const int32_t* __restrict__ big
     }
 }
 
-// kRows64: pipe scenes, with FP64 position rows to move too
-template <bool kRows64>
+// kRows64: pipe scenes, with FP64 position rows to move too.  kDense: tasks of
+// dense voxels have a list of their own.
+template <bool kRows64, bool kDense>
 __global__ void __launch_bounds__(512)
 k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict__ pid,
               const int32_t* __restrict__ tmp_pid, const int32_t* __restrict__ vstart,
@@ -420,10 +421,10 @@ k_rank_gather(int n, const int32_t* __restrict__ cell, const int32_t* __restrict
                 mine = !(vid & 16);       // the even voxel's first particle lists the pair
             }
         }
-        bool dense = tasks.dense_from && c >= tasks.dense_from;
-        if (dense && tasks.scenes) dense = tasks.scenes[scene_of(s, pbegin, n_scenes)].cap <= kListCap;
         if (!mine) {
-        } else if (dense)
+        } else if (kDense && c >= tasks.dense_from &&
+                   (!tasks.scenes ||
+                    tasks.scenes[scene_of(s, pbegin, n_scenes)].cap <= kListCap))
             tasks.dense_last[-atomicAdd(tasks.dense_count, 1)] = make_int2(vid, d);
         else
             tasks.list[atomicAdd(tasks.count, 1)] = make_int2(first, d);
@@ -500,10 +501,11 @@ cudaError_t launch_rank_gather(const Launch& L, const int32_t* cell, const int32
     // pipe's 262,144, before k_density_wc, 23 and 33).
     Launch next = L;
     if (tasks.tc_next && L.n <= 2048 * device_sm_count()) next.smem_share = 100;
-    return launch_chained(pos64 ? k_rank_gather<true> : k_rank_gather<false>, (L.n + b - 1) / b, b,
-                          next, L.n, cell, pid, tmp_pid, vstart, vcount, pos, vel, pos64, pos_out,
-                          vel_out, pid_out, pos64_out, tasks, L.big_voxel, slot, L.pbegin,
-                          L.n_scenes, L.step_limit, L.scene_step);
+    auto kernel = tasks.dense_last ? (pos64 ? k_rank_gather<true, true> : k_rank_gather<false, true>)
+                                   : (pos64 ? k_rank_gather<true, false> : k_rank_gather<false, false>);
+    return launch_chained(kernel, (L.n + b - 1) / b, b, next, L.n, cell, pid, tmp_pid, vstart,
+                          vcount, pos, vel, pos64, pos_out, vel_out, pid_out, pos64_out, tasks,
+                          L.big_voxel, slot, L.pbegin, L.n_scenes, L.step_limit, L.scene_step);
 }
 
 }  // namespace sphgb

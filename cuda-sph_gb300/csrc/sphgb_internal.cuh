@@ -473,6 +473,8 @@ __device__ inline void pipe_collide(double* p, double* v, const PipeView& P, uin
 // address must be 32-byte aligned).  In a gather, where the lanes of a warp
 // touch unrelated lines, an L1 pass costs per line touched, so one 32-byte
 // load of a force record costs half of two 16-byte loads.
+// For inlined code only: in a function of its own (noinline) nvcc 13.0 stored the
+// first of the eight elements and zeros.
 __device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -644,7 +646,7 @@ struct Launch {
     const double* pipe;         // device pipe table (may be null)
     bool pipe_scenes;           // some scene is in pipe mode
     int sort_block = kBlock;    // threads per block of the per-particle sort kernels
-    int big_voxel = 64;         // voxels above this many members are sorted per block
+    int big_voxel = 64;         // voxels above this many members go to the big-voxel sort
     int layout = 0;             // voxel tables: 0 all row-major, 1 all tiled, 2 mixed
     cudaStream_t stream;
     bool chained = true;        // see launch_chained
@@ -660,7 +662,7 @@ struct Launch {
 // Launches a kernel of the step so that its grid is set up while the kernel
 // before it on the stream drains (programmatic dependent launch); captured into
 // a graph, the edge is programmatic too.  Every such kernel starts with
-// grid_wait (or grid_wait_index) in every thread, so a kernel's completion
+// grid_wait in every thread, so a kernel's completion
 // implies the completion of all before it.
 template <class... P, class... A>
 cudaError_t launch_chained(void (*kernel)(P...), int blocks, int threads, const Launch& L,
@@ -696,7 +698,7 @@ cudaError_t launch_scatter(const Launch& L, const int32_t* cell, const int32_t* 
                            const int32_t* pid, const int32_t* vstart, const int32_t* vcount,
                            int32_t* tmp_pid, int32_t* big_list, int32_t* big_count);
 // voxels with more than Launch::big_voxel members (default kBigVoxel) get their
-// member ids sorted by one block each (the rank-gather then binary-searches
+// member ids sorted by a pass of their own (the rank-gather then binary-searches
 // them instead of counting); the threshold is never below kMinBigVoxel
 constexpr int kBigVoxel = 64;
 constexpr int kMinBigVoxel = 16;
@@ -720,9 +722,9 @@ constexpr int kTaskRun = 16;
 struct TaskLists {
     int2* list = nullptr;
     int32_t* count = nullptr;
-    int2* dense_last = nullptr;
+    int2* dense_last = nullptr;         // null: one list
     int32_t* dense_count = nullptr;
-    int dense_from = 0;  // 0: one list
+    int dense_from = 0;
     const SceneDev* scenes = nullptr;   // null: every scene is capped
     int pair_max = 0;    // 0: none
     bool tc_next = false;    // k_density_tc is the kernel after the rank-gather
